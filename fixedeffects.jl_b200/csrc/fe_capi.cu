@@ -140,6 +140,16 @@ bool is_pinned(const void* p) {
   return a.type == cudaMemoryTypeHost;
 }
 
+// the plan's own stream waits for what the default stream holds now
+int order_after_default(fe_plan* plan) {
+  cudaError_t e = cudaSuccess;
+  if (!plan->default_order)
+    e = cudaEventCreateWithFlags(&plan->default_order, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventRecord(plan->default_order, cudaStreamLegacy);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(plan->stream, plan->default_order, 0);
+  return e == cudaSuccess ? 0 : xfer_error("waiting for the default stream failed", e);
+}
+
 // Y: device matrix (cols == nullptr, leading dimension ld) or host columns.
 int solve_common(fe_plan* plan, void* Y, void* const* cols, int32_t dtype, int64_t ncols,
                  int64_t ld, int32_t precision, double tol, int64_t maxiter,
@@ -240,6 +250,9 @@ int solve_common(fe_plan* plan, void* Y, void* const* cols, int32_t dtype, int64
   } else {
     rq.Y = Y;
     rq.ld = ld;
+    // a plan on its own stream does not order itself after the work that the
+    // caller has queued on the default stream (its own stream is non-blocking)
+    if (plan->own_stream && (st = order_after_default(plan))) return st;
   }
   st = fe::solve(plan, rq);
   if (st) return st;

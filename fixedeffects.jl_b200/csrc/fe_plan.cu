@@ -842,6 +842,7 @@ int plan_destroy(fe_plan* pl) {
   }
   if (pl->host_pinned) cudaFreeHost(pl->host_pinned);
   if (pl->noalloc_order) cudaEventDestroy(pl->noalloc_order);
+  if (pl->default_order) cudaEventDestroy(pl->default_order);
   if (pl->ring_up) cudaFreeHost(pl->ring_up);
   if (pl->ring_down) cudaFreeHost(pl->ring_down);
   for (auto& g : pl->graphs)

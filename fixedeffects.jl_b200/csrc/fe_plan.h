@@ -225,6 +225,8 @@ struct fe_plan {
   void* host_pinned = nullptr;  // small pinned staging for counters
   // fe_plan_scales_noalloc on a caller stream: orders it after the plan's stream
   cudaEvent_t noalloc_order = nullptr;
+  // device-buffer solves on the plan's own stream: orders it after the default stream
+  cudaEvent_t default_order = nullptr;
   // pinned staging rings of pageable host-buffer solves (fe_staging.cu)
   void* ring_up = nullptr;
   void* ring_down = nullptr;
