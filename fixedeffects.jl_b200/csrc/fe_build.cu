@@ -559,15 +559,17 @@ int plan_build_device(fe_plan* pl, const int64_t* const* refs, const int64_t* n_
   pl->d_refs.resize(K);
   pl->d_perm.resize(K);
   pl->d_key.resize(K);
+  pl->d_off.resize(K);
   pl->perm_identity.assign(K, false);
   pl->seg_off.assign(K, {});
   pl->seg_len.assign(K, 0);
-  DevBuf flag, off;
+  DevBuf flag;
   st = flag.ensure(4);
   if (st) return st;
   for (int k = 0; k < K; ++k) {
     const int64_t nb = pl->nlev[k] + 1;  // levels + the null level (last)
     st = pl->d_refs[k].ensure((size_t)std::max<int64_t>(N, 1) * 4);
+    DevBuf& off = pl->d_off[k];
     if (!st) st = off.ensure((size_t)(nb + 1) * 4);
     if (st) return st;
     int32_t* rs = pl->d_refs[k].as<int32_t>();

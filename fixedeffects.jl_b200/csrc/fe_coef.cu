@@ -1,0 +1,584 @@
+// fe_coef.cu -- plan data, row kernels and driver of the coefficient-side
+// solve (fe_coef.h; the solve kernel itself is fe_coef.cuh).
+#include "fe_coef.h"
+
+#include <algorithm>
+#include <cstring>
+
+#include "fe_prof.h"
+
+namespace fe {
+
+static inline unsigned grid1(int64_t n, int b = 256) { return (unsigned)((n + b - 1) / b); }
+
+// ---------------------------------------------------------------------------
+// plan data
+// ---------------------------------------------------------------------------
+static __global__ void k_take_i(const int32_t* __restrict__ src, const int32_t* __restrict__ perm,
+                                int32_t* __restrict__ dst, int64_t n) {
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < n) dst[q] = src[perm ? perm[q] : q];
+}
+// out[q] = product of sw^2 and of up to four interactions, at position q
+struct CoefProduct {
+  const double* sw;
+  const double* x[kCoefMaxFE + 1];
+};
+static __global__ void k_product(const CoefProduct a, const int32_t* __restrict__ perm,
+                                 double* __restrict__ dst, int64_t n) {
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  const int64_t i = perm ? perm[q] : q;
+  double v = 1.0;
+  if (a.sw) v = a.sw[i] * a.sw[i];
+#pragma unroll
+  for (int g = 0; g <= kCoefMaxFE; ++g)
+    if (a.x[g]) v *= a.x[g][i];
+  dst[q] = v;
+}
+static __global__ void k_lev_primary(const double* __restrict__ scale, double* __restrict__ lev,
+                                     int64_t n) {
+  const int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (l < n) lev[l] = scale[l] * scale[l];
+}
+static __global__ void k_lev_other(const double* __restrict__ scale,
+                                   const double* __restrict__ abs_scale, double* __restrict__ lev,
+                                   int64_t n) {
+  const int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (l >= n) return;
+  const double j = scale[l], s = abs_scale[l];
+  lev[4 * l] = j > 0 ? 1.0 / (j * j) : 0.0;
+  lev[4 * l + 1] = s * s;
+  lev[4 * l + 2] = s > 0 ? 1.0 / (s * s) : 0.0;
+  lev[4 * l + 3] = 0.0;
+}
+
+static int coef_plan(fe_plan* pl) {
+  if (!pl->coef) pl->coef = std::make_shared<CoefPlan>();
+  CoefPlan& cp = *pl->coef;
+  cudaStream_t s = pl->stream;
+  const int kp = pl->primary;
+  const int64_t N = pl->N;
+  int st = 0;
+  if (!cp.built) {
+    cp.nf = 0;
+    cp.rows = 0;
+    for (int k = 0; k < pl->K; ++k)
+      if (k != kp) {
+        cp.fe[cp.nf] = k;
+        cp.base[cp.nf] = cp.rows;
+        cp.rows += pl->nlev[k];
+        ++cp.nf;
+      }
+    for (int f = 0; f < cp.nf; ++f) {
+      const int32_t* perm = pl->dev.perm[cp.fe[f]];
+      if ((st = cp.zi[f].ensure((size_t)N * 4))) return st;
+      k_take_i<<<grid1(N), 256, 0, s>>>(pl->dev.refs[kp], perm, cp.zi[f].as<int32_t>(), N);
+      for (int g = 0; g < cp.nf; ++g) {
+        if (g == f) continue;
+        if ((st = cp.gi[f][g].ensure((size_t)N * 4))) return st;
+        k_take_i<<<grid1(N), 256, 0, s>>>(pl->dev.refs[cp.fe[g]], perm, cp.gi[f][g].as<int32_t>(), N);
+      }
+      FE_CK(cudaGetLastError());
+    }
+    cp.built = true;
+  }
+  if (!cp.weights_built) {
+    for (auto& w : cp.wt) w.second.filled = false;
+    for (int f = 0; f <= cp.nf; ++f) {
+      const int k = f < cp.nf ? cp.fe[f] : kp;
+      const int64_t n = pl->nlev[k];
+      if ((st = cp.lev[f].ensure((size_t)std::max<int64_t>(n, 1) * (f < cp.nf ? 32 : 8)))) return st;
+      if (n > 0) {
+        if (f < cp.nf)
+          k_lev_other<<<grid1(n), 256, 0, s>>>(pl->d_scale_d[k].as<double>(),
+                                               pl->d_abs_scale_d[k].as<double>(),
+                                               cp.lev[f].as<double>(), n);
+        else
+          k_lev_primary<<<grid1(n), 256, 0, s>>>(pl->d_scale_d[k].as<double>(),
+                                                 cp.lev[f].as<double>(), n);
+      }
+      FE_CK(cudaGetLastError());
+    }
+    cp.weights_built = true;
+  }
+  return 0;
+}
+
+// The product of w (bit 0) and of the interactions of the FE slots whose bit
+// 1 + slot is set, in the order of FE slot f; null: all 1.
+static int coef_weights(fe_plan* pl, int f, int mask, const double** out) {
+  CoefPlan& cp = *pl->coef;
+  CoefProduct p;
+  memset(&p, 0, sizeof(p));
+  int m = 0, eff = 0;
+  if ((mask & 1) && pl->weighted) {
+    p.sw = pl->d_sw_sorted.as<double>();
+    eff |= 1;
+  }
+  for (int g = 0; g <= cp.nf; ++g) {
+    const int k = g < cp.nf ? cp.fe[g] : pl->primary;
+    if (!((mask >> (1 + g)) & 1) || !pl->interacted[k]) continue;
+    p.x[m++] = pl->d_inter_sorted[k].as<double>();
+    eff |= 2 << g;
+  }
+  *out = nullptr;
+  if (!eff) return 0;
+  CoefPlan::Weights& w = cp.wt[{f, eff}];
+  const int st = w.buf.ensure((size_t)pl->N * 8);
+  if (st) return st;
+  if (!w.filled) {
+    const int k = f < cp.nf ? cp.fe[f] : pl->primary;
+    k_product<<<grid1(pl->N), 256, 0, pl->stream>>>(p, pl->dev.perm[k], w.buf.as<double>(), pl->N);
+    FE_CK(cudaGetLastError());
+    w.filled = true;
+  }
+  *out = w.buf.as<double>();
+  return 0;
+}
+
+// Work items: consecutive levels packed into windows, longer levels cut into
+// pieces.  A warp has 32 / (CL << rlog) teams; rlog is the smallest with which
+// a round of levels of mean length fits a window, and an item holds whole
+// rounds, so that no team idles for want of a level.  Levels longer than a
+// quarter of a warp's share of the positions are cut, so that few long levels
+// still fill the GPU evenly (but not below 4 steps of a warp: a level of
+// several pieces costs a handshake and a norm slot).
+static int coef_items(fe_plan* pl, int C, int window, CoefPlan::Items** out) {
+  CoefPlan& cp = *pl->coef;
+  std::unique_ptr<CoefPlan::Items>& slot = cp.items[{C, window}];
+  if (slot) {
+    *out = slot.get();
+    return 0;
+  }
+  std::unique_ptr<CoefPlan::Items> its(new CoefPlan::Items());
+  int sms = 148;
+  FE_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device));
+  const int cl = C >= 4 ? C / 4 : 1;
+  const int64_t share = pl->N / std::max<int64_t>(1, (int64_t)sms * kCoefWarps);
+  const int64_t psz = std::max<int64_t>(4 * (32 / cl), std::min<int64_t>(16384, share / 4));
+  std::vector<CoefItem> whole, items;
+  std::vector<CoefPiece> pcs;
+  for (int f = 0; f <= cp.nf; ++f) {
+    const int k = f < cp.nf ? cp.fe[f] : pl->primary;
+    const std::vector<int64_t>& off = pl->seg_off[k];
+    const int64_t nl = pl->nlev[k];
+    const double avg = nl > 0 ? std::max(1.0, (double)pl->seg_len[k] / (double)nl) : 1.0;
+    int rlog = 0;
+    while ((cl << rlog) < 32 && avg * (32 / (cl << rlog)) > window) ++rlog;
+    const int nt = 32 / (cl << rlog);
+    const int rounds = std::max(1, (int)(window / (avg * nt)));
+    const int cap = std::min(32, nt * rounds);
+    its->rlog[f] = rlog;
+    if (f == cp.nf) its->multi_p = its->nmulti;
+    its->piece0[f] = its->pieces;
+    whole.clear();
+    items.clear();
+    pcs.clear();
+    int64_t l0 = 0;  // first level of the open item
+    auto close = [&](int64_t l) {
+      if (l > l0)
+        whole.push_back({(uint32_t)off[(size_t)l0], (uint32_t)off[(size_t)l], (int32_t)l0,
+                         (int32_t)(l - l0)});
+      l0 = l;
+    };
+    for (int64_t l = 0; l < nl; ++l) {
+      const int64_t b = off[(size_t)l], e = off[(size_t)l + 1], n = e - b;
+      if (n > window) {
+        close(l);
+        l0 = l + 1;
+        const int64_t np = (n + psz - 1) / psz, sz = (n + np - 1) / np;
+        const int32_t first = (int32_t)pcs.size();
+        for (int64_t i = 0; i < np; ++i) {
+          items.push_back({(uint32_t)(b + i * sz), (uint32_t)std::min(b + (i + 1) * sz, e),
+                           (int32_t)l, -1 - (int32_t)pcs.size()});
+          pcs.push_back({first, (int32_t)np, its->nmulti, 0});
+        }
+        if (np > 1) ++its->nmulti;
+        continue;
+      }
+      if (l - l0 == cap || e - off[(size_t)l0] > window) close(l);
+    }
+    close(nl);
+    items.insert(items.end(), whole.begin(), whole.end());
+    its->n[f] = (int64_t)items.size();
+    its->pieces += (int32_t)pcs.size();
+    int st = its->dev[f].ensure(std::max<size_t>(items.size(), 1) * sizeof(CoefItem));
+    if (!st) st = its->piece[f].ensure(std::max<size_t>(pcs.size(), 1) * sizeof(CoefPiece));
+    if (st) return st;
+    if (!items.empty())
+      FE_CK(cudaMemcpyAsync(its->dev[f].p, items.data(), items.size() * sizeof(CoefItem),
+                            cudaMemcpyHostToDevice, pl->stream));
+    if (!pcs.empty())
+      FE_CK(cudaMemcpyAsync(its->piece[f].p, pcs.data(), pcs.size() * sizeof(CoefPiece),
+                            cudaMemcpyHostToDevice, pl->stream));
+    FE_CK(cudaStreamSynchronize(pl->stream));  // the host lists are reused
+  }
+  const int st = its->cnt.ensure((size_t)std::max(its->nmulti, 1) * 4);
+  if (st) return st;
+  slot = std::move(its);
+  *out = slot.get();
+  return 0;
+}
+
+// ---------------------------------------------------------------------------
+// rows: host layout <-> sorted [N][C] rows
+// ---------------------------------------------------------------------------
+// As k_load / k_unload of fe_solve_impl.cuh, without weights and in FP32, the
+// caller's type: half the bytes of an FP64 row copy.
+constexpr int kRowElems = 2048;  // elements per CTA
+template <int C>
+__global__ void __launch_bounds__(256) k_rows_in(const float* __restrict__ Y, int64_t ld, int64_t col0,
+                                                 int ncols, const int32_t* __restrict__ dst,
+                                                 float* __restrict__ B, int64_t N) {
+  constexpr int R = kRowElems / C, PER = kRowElems / 256;
+  __shared__ float tile[R][C + 1];
+  const int64_t i0 = (int64_t)blockIdx.x * R;
+  float v[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = threadIdx.x + u * 256;
+    const int j = e / R, r = e % R;
+    v[u] = (i0 + r < N && j < ncols) ? Y[i0 + r + (col0 + j) * ld] : 0.f;
+  }
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = threadIdx.x + u * 256;
+    tile[e % R][e / R] = v[u];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = threadIdx.x + u * 256;
+    const int r = e / C, j = e % C;
+    if (i0 + r < N) B[(int64_t)__ldg(dst + i0 + r) * C + j] = tile[r][j];
+  }
+}
+// tiles of 1 or 2 columns: gathered through the inverse permutation, so that
+// the rows, shorter than a sector, are written in order
+template <int C>
+__global__ void __launch_bounds__(256) k_rows_gather(const float* __restrict__ Y, int64_t ld,
+                                                     int64_t col0, int ncols,
+                                                     const int32_t* __restrict__ src,
+                                                     float* __restrict__ B, int64_t N) {
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= N) return;
+  const int64_t i = src[q];
+#pragma unroll
+  for (int j = 0; j < C; ++j) B[q * C + j] = j < ncols ? Y[i + (col0 + j) * ld] : 0.f;
+}
+template <int C>
+__global__ void __launch_bounds__(256) k_rows_out(const float* __restrict__ B, int64_t ld, int64_t col0,
+                                                  int ncols, const int32_t* __restrict__ dst,
+                                                  float* __restrict__ Y, int64_t N,
+                                                  const uint32_t* __restrict__ bar) {
+  constexpr int R = kRowElems / C, PER = kRowElems / 256;
+  __shared__ float tile[R][C + 1];
+  if (bar[2]) return;  // the caller takes the row-side path
+  const int64_t i0 = (int64_t)blockIdx.x * R;
+  float v[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = threadIdx.x + u * 256;
+    const int r = e / C, j = e % C;
+    v[u] = i0 + r < N ? B[(int64_t)__ldg(dst + i0 + r) * C + j] : 0.f;
+  }
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = threadIdx.x + u * 256;
+    tile[e / C][e % C] = v[u];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = threadIdx.x + u * 256;
+    const int j = e / R, r = e % R;
+    if (i0 + r < N && j < ncols) Y[i0 + r + (col0 + j) * ld] = tile[r][j];
+  }
+}
+
+// r = y - A_r x - A_p (zb - z), in place on the sorted rows.  An observation
+// of weight 0 gets NaN, as dividing its weighted residual by sqrt(w) does
+// (src/AbstractFixedEffectSolver.jl:62-66).
+struct CoefResid {
+  const int32_t* refp;
+  const int32_t* gi[kCoefMaxFE];
+  const double* tab[kCoefMaxFE];
+  const double* xg[kCoefMaxFE];
+  const double *xp, *w, *zb, *z;
+  int nf;
+};
+template <int C>
+__global__ void __launch_bounds__(256) k_rows_resid(const CoefResid a, float* __restrict__ B, int64_t N,
+                                                    const uint32_t* __restrict__ bar) {
+  constexpr int VEC = C >= 2 ? 2 : 1, CL = C / VEC;
+  if (bar[2]) return;
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const int64_t q = e / CL;
+  if (q >= N) return;
+  const int j0 = (int)(e % CL) * VEC;
+  const int64_t lp = __ldg(a.refp + q);
+  const double xp = a.xp ? __ldg(a.xp + q) : 1.0;
+  double fit[VEC], y[VEC];
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) {
+    fit[v] = xp * (__ldg(a.zb + lp * C + j0 + v) - __ldg(a.z + lp * C + j0 + v));
+    y[v] = (double)B[q * C + j0 + v];
+  }
+#pragma unroll
+  for (int g = 0; g < kCoefMaxFE; ++g) {
+    if (g >= a.nf) break;
+    const double xg = a.xg[g] ? __ldg(a.xg[g] + q) : 1.0;
+    const double* t = a.tab[g] + (int64_t)__ldg(a.gi[g] + q) * C + j0;
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) fit[v] += xg * __ldg(t + v);
+  }
+  const bool zero = a.w && __ldg(a.w + q) == 0.0;
+#pragma unroll
+  for (int v = 0; v < VEC; ++v)
+    B[q * C + j0 + v] = zero ? (float)nan("") : (float)(y[v] - fit[v]);
+}
+
+template <int C>
+static int rows_in(fe_plan* pl, const SolveReq& rq, int64_t col0, int ncols, float* B) {
+  if (C <= 2)
+    k_rows_gather<C><<<grid1(pl->N), 256, 0, pl->stream>>>(
+        (const float*)rq.Y, rq.ld, col0, ncols, pl->d_obs_src.as<int32_t>(), B, pl->N);
+  else
+    k_rows_in<C><<<grid1(pl->N, kRowElems / C), 256, 0, pl->stream>>>(
+        (const float*)rq.Y, rq.ld, col0, ncols, pl->d_obs_dst.as<int32_t>(), B, pl->N);
+  FE_CK(cudaGetLastError());
+  return 0;
+}
+template <int C>
+static int rows_out(fe_plan* pl, const SolveReq& rq, int64_t col0, int ncols, float* B,
+                    const CoefResid& r, const uint32_t* bar, double rbytes, double ubytes) {
+  constexpr int CL = C >= 2 ? C / 2 : 1;
+  {
+    ProfScope ps(pl, "resid", rbytes);
+    k_rows_resid<C><<<grid1(pl->N * CL), 256, 0, pl->stream>>>(r, B, pl->N, bar);
+    FE_CK(cudaGetLastError());
+  }
+  ProfScope ps(pl, "unload", ubytes);
+  k_rows_out<C><<<grid1(pl->N, kRowElems / C), 256, 0, pl->stream>>>(
+      B, rq.ld, col0, ncols, pl->d_obs_dst.as<int32_t>(), (float*)rq.Y, pl->N, bar);
+  FE_CK(cudaGetLastError());
+  return 0;
+}
+
+// ---------------------------------------------------------------------------
+// driver
+// ---------------------------------------------------------------------------
+// Mixed-precision residual solves of FP32 columns on plans whose primary FE is
+// absorbed, with at most kCoefMaxFE other FEs, unless an option names a kernel
+// of the row-side loop.  (FP64 columns keep the row-side iteration: theirs are
+// returned unrounded, so another iteration would show in them at the level of
+// the tolerance.  Every further FE adds a gather per position to every other
+// FE's pass, so the passes grow with the square of their number.)
+bool coef_takes(const fe_plan* pl, const SolveReq& rq, int C) {
+  return C <= kCoefMaxCols && rq.precision == 1 && rq.dtype == 1 && rq.residuals && pl->absorbable && pl->opt_absorb != 0 &&
+         pl->opt_abs_scale != 0 && pl->nprob == 1 && !pl->xchg && pl->N > 0 &&
+         pl->K - 1 <= kCoefMaxFE && pl->perm_identity[pl->primary] && pl->opt_exdm != 0 &&
+         pl->opt_exdm_pipe < 0 && pl->opt_firm_atomic == 0 && pl->opt_fused_resid != 1 &&
+         pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0;
+}
+
+static const void* kernel_of(int C, int nf, int w, size_t* smem) {
+  switch (C) {
+    case 1: *smem = coef_smem_bytes<1>(nf, w); return coef_kernel<1>(nf, w);
+    case 2: *smem = coef_smem_bytes<2>(nf, w); return coef_kernel<2>(nf, w);
+    case 4: *smem = coef_smem_bytes<4>(nf, w); return coef_kernel<4>(nf, w);
+    default: *smem = coef_smem_bytes<8>(nf, w); return coef_kernel<8>(nf, w);
+  }
+}
+
+#define FE_COEF_C(C, CALL)          \
+  switch (C) {                      \
+    case 1: { constexpr int W = 1; CALL; break; }   \
+    case 2: { constexpr int W = 2; CALL; break; }   \
+    case 4: { constexpr int W = 4; CALL; break; }   \
+    default: { constexpr int W = 8; CALL; break; }  \
+  }
+
+int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int ncols,
+                    std::vector<Inst>& out, int* done) {
+  NvtxRange nv("fe: tile (coefficient side)");
+  *done = 0;
+  int st = coef_plan(pl);
+  if (st) return st;
+  CoefPlan& cp = *pl->coef;
+  const int kp = pl->primary, nf = cp.nf;
+  const int64_t N = pl->N;
+  const size_t es = 4, rc = (size_t)C * 8;
+  const size_t pn = (size_t)std::max<int64_t>(pl->nlev[kp], 1), rn = (size_t)std::max<int64_t>(cp.rows, 1);
+  int weights = pl->weighted ? 1 : 0;
+  for (int k = 0; k < pl->K; ++k)
+    if (pl->interacted[k]) weights = 2;
+  CoefPlan::Items* its = nullptr;
+  if ((st = coef_items(pl, C, coef_window(nf, weights), &its))) return st;
+  size_t smem = 0;
+  const void* kern = kernel_of(C, nf, weights, &smem);
+  int sms = 148;
+  FE_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device));
+  // opt-in shared memory, once per kernel and device
+  static PerDeviceOnce attr_set[4][9];
+  const int ci = C == 1 ? 0 : C == 2 ? 1 : C == 4 ? 2 : 3;
+  PerDeviceOnce& once = attr_set[ci][(nf - 1) * 3 + weights];
+  if (once.needed(pl->device)) {
+    FE_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    once.done(pl->device);
+  }
+  if (!its->occ || its->occ_w != weights) {
+    int o = 0;
+    FE_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, kCoefThreads, smem));
+    if (o < 1) return 0;
+    its->occ = o;
+    its->occ_w = weights;
+  }
+  // small problems take few CTAs (a barrier costs the more the more arrive)
+  const int64_t grid = std::max<int64_t>(
+      1, std::min<int64_t>((int64_t)its->occ * sms, (N * ((C + 3) / 4) + 511) / 512));
+  if ((st = cp.y.ensure((size_t)N * C * es))) return st;
+  if ((st = cp.zb.ensure(pn * rc))) return st;
+  if ((st = cp.z.ensure(pn * rc))) return st;
+  for (DevBuf* b : {&cp.ta, &cp.tb, &cp.h, &cp.hb, &cp.xx, &cp.c})
+    if ((st = b->ensure(rn * rc))) return st;
+  if ((st = cp.part.ensure((size_t)2 * 3 * grid * rc))) return st;
+  if ((st = cp.ppart.ensure((size_t)std::max(its->pieces, 1) * rc))) return st;
+  if ((st = cp.mnrm.ensure((size_t)3 * std::max(its->nmulti, 1) * rc))) return st;
+  if ((st = cp.bar.ensure(64 + (size_t)C * sizeof(Inst)))) return st;
+  CoefArgs a;
+  memset(&a, 0, sizeof(a));
+  for (int f = 0; f <= nf; ++f) {
+    CoefSide& sd = f < nf ? a.f[f] : a.p;
+    const int k = f < nf ? cp.fe[f] : kp;
+    sd.off = pl->d_off[k].as<int32_t>();
+    sd.perm = pl->dev.perm[k];
+    // the weight arrays of this order, each distinct one staged once
+    int nd = 0;
+    const auto slot = [&](int mask, int32_t* out) -> int {
+      const double* p = nullptr;
+      const int e = coef_weights(pl, f, mask, &p);
+      if (e) return e;
+      *out = -1;
+      for (int i = 0; i < nd && p; ++i)
+        if (sd.d[i] == p) *out = i;
+      if (p && *out < 0) {
+        *out = nd;
+        sd.d[nd++] = p;
+      }
+      return 0;
+    };
+    const int own = 2 << f, prim = 2 << nf;
+    int m = 0;
+    for (int g = 0; g < nf; ++g) {
+      if (g == f) continue;
+      sd.gi[m] = f < nf ? cp.gi[f][g].as<int32_t>() : pl->dev.refs[cp.fe[g]];
+      sd.gb[m] = cp.base[g];
+      const int mask = f < nf ? 1 | own | (2 << g) : nf == 1 ? 1 | prim | (2 << g) : 2 << g;
+      if ((st = slot(mask, &sd.slot_g[m]))) return st;
+      ++m;
+    }
+    sd.slot_w = sd.slot_n = -1;
+    if ((f < nf || nf > 1) && (st = slot(f < nf ? 1 | own | prim : 1 | prim, &sd.slot_w))) return st;
+    if (f == nf && nf > 1 && (st = slot(1, &sd.slot_n))) return st;
+    if ((st = coef_weights(pl, f, 1, &sd.dw))) return st;
+    if ((st = coef_weights(pl, f, f < nf ? 1 | own : 1 | prim, &sd.dwx))) return st;
+    if (f < nf) {
+      sd.zi = cp.zi[f].as<int32_t>();
+      sd.base = cp.base[f];
+    }
+    sd.lev = cp.lev[f].as<double>();
+    sd.items = its->dev[f].as<CoefItem>();
+    sd.pieces = its->piece[f].as<CoefPiece>();
+    sd.nitems = (int32_t)its->n[f];
+    sd.piece0 = its->piece0[f];
+    sd.n = (int32_t)pl->nlev[k];
+    sd.rlog = its->rlog[f];
+    sd.npos = (uint32_t)N;
+  }
+  a.y = cp.y.as<float>();
+  a.ncols = ncols;
+  a.zb = cp.zb.as<double>();
+  a.z = cp.z.as<double>();
+  a.ta = cp.ta.as<double>();
+  a.tb = cp.tb.as<double>();
+  a.h = cp.h.as<double>();
+  a.hb = cp.hb.as<double>();
+  a.x = cp.xx.as<double>();
+  a.c = cp.c.as<double>();
+  a.part = cp.part.as<double>();
+  a.ppart = cp.ppart.as<double>();
+  a.mnrm = cp.mnrm.as<double>();
+  a.nmulti = its->nmulti;
+  a.multi_p = its->multi_p;
+  a.pcnt = its->cnt.as<int32_t>();
+  a.bar = cp.bar.as<uint32_t>();
+  a.inst = reinterpret_cast<Inst*>(static_cast<char*>(cp.bar.p) + 64);
+  a.tol = rq.tol;
+  a.theta = pl->opt_inner_theta;
+  // the inner solves run in FP64: the floor of the option's FP32 value falls
+  // by the ratio of the roundings
+  a.rho = pl->opt_inner_rho * 1e-6;
+  a.maxiter = rq.maxiter - 1;
+  a.max_rounds = pl->opt_max_rounds;
+  FE_CK(cudaMemsetAsync(cp.bar.p, 0, 64, pl->stream));
+  FE_CK(cudaMemsetAsync(its->cnt.p, 0, its->cnt.bytes, pl->stream));
+  {
+    ProfScope ps(pl, "load", (double)N * (ncols + C) * es);
+    FE_COEF_C(C, (st = rows_in<W>(pl, rq, col0, ncols, cp.y.as<float>())));
+    if (st) return st;
+  }
+  {
+    ProfScope ps(pl, "coef_solve", 0.0);
+    void* params[] = {&a};
+    FE_CK(cudaLaunchCooperativeKernel(kern, dim3((unsigned)grid), dim3(kCoefThreads), params, smem,
+                                      pl->stream));
+  }
+  CoefResid r;
+  memset(&r, 0, sizeof(r));
+  r.refp = pl->dev.refs[kp];
+  r.xp = pl->interacted[kp] ? pl->d_inter_sorted[kp].as<double>() : nullptr;
+  r.w = pl->weighted ? pl->d_sw_sorted.as<double>() : nullptr;
+  r.zb = a.zb;
+  r.z = a.z;
+  r.nf = nf;
+  for (int g = 0; g < nf; ++g) {
+    r.gi[g] = a.p.gi[g];
+    r.xg[g] = pl->interacted[cp.fe[g]] ? pl->d_inter_sorted[cp.fe[g]].as<double>() : nullptr;
+    r.tab[g] = a.x + cp.base[g] * C;
+  }
+  const double meta = (double)N * (4.0 * pl->K + (pl->weighted ? 8 : 0));
+  const double rbytes = meta + (double)N * C * 2 * es + (double)pn * rc * 2 + (double)rn * rc;
+  const double ubytes = (double)N * (ncols + C) * es;
+  FE_COEF_C(C, (st = rows_out<W>(pl, rq, col0, ncols, cp.y.as<float>(), r, a.bar, rbytes, ubytes)));
+  if (st) return st;
+  std::vector<char> res(64 + (size_t)C * sizeof(Inst));
+  FE_CK(cudaMemcpyAsync(res.data(), cp.bar.p, res.size(), cudaMemcpyDeviceToHost, pl->stream));
+  FE_CK(cudaStreamSynchronize(pl->stream));
+  uint32_t bar[3];
+  memcpy(bar, res.data(), sizeof(bar));
+  if (bar[2]) return prof_flush(pl);
+  out.resize((size_t)C);
+  memcpy(out.data(), res.data() + 64, (size_t)C * sizeof(Inst));
+  // bytes of the solve kernel: per iteration (the longest column's) the index
+  // and weight arrays of every order, one gathered z row per position of the
+  // other FEs, the z rows written, the coefficient vectors
+  int64_t iters = 0, rounds = 0;
+  for (const Inst& s : out) {
+    iters = std::max(iters, s.iter_total);
+    rounds = std::max<int64_t>(rounds, s.outer_rounds);
+  }
+  double per = 0.0;
+  for (int f = 0; f <= nf; ++f) {
+    const CoefSide& sd = f < nf ? a.f[f] : a.p;
+    per += (double)N * 4.0 * nf + (f < nf ? (double)N * rc : (double)pn * rc);
+    for (const double* d : sd.d) per += d ? (double)N * 8.0 : 0.0;
+  }
+  pl->prof.bytes_per_launch["coef_solve"] =
+      (per + 9.0 * rn * rc) * (double)(iters + rounds) + (double)N * C * es * (1 + nf) + (double)N * rc * nf;
+  *done = 1;
+  return prof_flush(pl);
+}
+
+}  // namespace fe

@@ -16,6 +16,7 @@
 #include <string>
 #include <vector>
 
+#include "fe_coef.h"
 #include "fe_kernels.cuh"
 #include "fe_plan.h"
 
@@ -372,6 +373,7 @@ int plan_update_weights(fe_plan* pl, const double* weights) {
   for (auto& g : pl->graphs)
     if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
   pl->graphs.clear();
+  if (pl->coef) pl->coef->weights_built = false;
   pl->weighted = weights != nullptr;
   if (weights) {
     DevBuf w;

@@ -146,6 +146,8 @@ struct LoopGraph {
   size_t key = 0;  // fingerprint of everything the captured launches use
 };
 
+struct CoefPlan;  // fe_coef.h
+
 struct Profile {
   bool on = false;
   std::map<std::string, KernelStat> stats;
@@ -182,6 +184,7 @@ struct fe_plan {
   // device integer plan
   fe::DevBuf d_obs_src, d_obs_dst;     // sorted -> original, original -> sorted
   std::vector<fe::DevBuf> d_refs, d_perm, d_key;
+  std::vector<fe::DevBuf> d_off;  // per FE: level-order offsets (levels, then the null level)
   std::vector<bool> perm_identity;
   // device weights/interaction/preconditioner
   fe::DevBuf d_sw_orig, d_sw_sorted;
@@ -220,6 +223,7 @@ struct fe_plan {
   std::string tune_signature;   // plan shape, key of the persisted tuning cache
 
   std::map<int, std::unique_ptr<fe::ItemSet>> items;  // by C
+  std::shared_ptr<fe::CoefPlan> coef;  // coefficient-side solves (fe_coef.cu)
   fe::Workspace ws;
   fe::Profile prof;
   void* host_pinned = nullptr;  // small pinned staging for counters

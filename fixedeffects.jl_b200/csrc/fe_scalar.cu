@@ -10,138 +10,9 @@
 #include <cuda_runtime.h>
 
 #include "fe_internal.h"
+#include "fe_lsmr.cuh"
 
 namespace fe {
-
-// Kernel coefficients of a stopped instance: the expand keeps U
-// (U <- 0*(A v) + 1*U) and the P-side update is skipped (upd_mode 0, no v).
-__device__ static void deactivate(Inst& s) {
-  s.active = 0;
-  s.ex_av = 0.0;
-  s.ex_au = 1.0;
-  s.upd_mode = 0;
-  s.do_v = 0;
-}
-
-__device__ static void lsmr_test(Inst& s) {
-  // src/utils/lsmr.jl:188-215
-  const double test1 = s.normr / s.normb;
-  const double test2 = s.normAr / (s.normA * s.normr);
-  const double test3 = 1.0 / s.condA;
-  const double t1 = test1 / (1.0 + s.normA * s.normx / s.normb);
-  const double rtol = s.btol + s.atol * s.normA * s.normx / s.normb;
-  int istop = 0;
-  if (s.iter >= s.maxiter) istop = 7;
-  else if (1.0 + test3 <= 1.0) istop = 6;
-  else if (1.0 + test2 <= 1.0) istop = 5;
-  else if (1.0 + t1 <= 1.0) istop = 4;
-  else if (test3 <= s.ctol) istop = 3;
-  else if (test2 <= s.atol) istop = 2;
-  else if (test1 <= rtol) istop = 1;
-  if (!istop && s.mode_inner) {
-    // inner solve of the mixed mode: stop once the FP64 outer test is
-    // expected to pass, or once normAr fell by inner_rho (the FP32 floor)
-    const double nAt = sqrt(s.normA2_prev + s.normA * s.normA);
-    if (s.normAr <= s.inner_theta_tol * nAt * s.normr || s.normAr <= s.inner_rho * s.normAr0)
-      istop = 2;
-  }
-  s.istop = istop;
-}
-
-__device__ static void lsmr_rotate(Inst& s) {
-  // src/utils/lsmr.jl:113-186, lambda = 0
-  const double lambda = 0.0;
-  const double alphahat = sqrt(s.alphabar * s.alphabar + lambda * lambda);
-  const double chat = s.alphabar / alphahat;
-  const double shat = lambda / alphahat;
-  const double rhoold = s.rho;
-  s.rho = sqrt(alphahat * alphahat + s.beta * s.beta);
-  const double c = alphahat / s.rho;
-  const double sn = s.beta / s.rho;
-  const double thetanew = sn * s.alpha;
-  s.alphabar = c * s.alpha;
-  const double rhobarold = s.rhobar;
-  const double zetaold = s.zeta;
-  const double thetabar = s.sbar * s.rho;
-  const double rhotemp = s.cbar * s.rho;
-  s.rhobar = sqrt((s.cbar * s.rho) * (s.cbar * s.rho) + thetanew * thetanew);
-  s.cbar = s.cbar * s.rho / s.rhobar;
-  s.sbar = thetanew / s.rhobar;
-  s.zeta = s.cbar * s.zetabar;
-  s.zetabar = -s.sbar * s.zetabar;
-  // coefficients of the (deferred) vector update, lsmr.jl:138-142
-  s.c1 = -thetabar * s.rho / (rhoold * rhobarold);
-  s.c2 = s.zeta / (s.rho * s.rhobar);
-  s.c3 = -thetanew / s.rho;
-  // estimate of ||r||
-  const double betaacute = chat * s.betadd;
-  const double betacheck = -shat * s.betadd;
-  const double betahat = c * betaacute;
-  s.betadd = -sn * betaacute;
-  const double thetatildeold = s.thetatilde;
-  const double rhotildeold = sqrt(s.rhodold * s.rhodold + thetabar * thetabar);
-  const double ctildeold = s.rhodold / rhotildeold;
-  const double stildeold = thetabar / rhotildeold;
-  s.thetatilde = stildeold * s.rhobar;
-  s.rhodold = ctildeold * s.rhobar;
-  s.betad = -stildeold * s.betad + ctildeold * betahat;
-  s.tautildeold = (zetaold - thetatildeold * s.tautildeold) / rhotildeold;
-  const double taud = (s.zeta - s.thetatilde * s.tautildeold) / s.rhodold;
-  s.d = s.d + betacheck * betacheck;
-  s.normr = sqrt(s.d + (s.betad - taud) * (s.betad - taud) + s.betadd * s.betadd);
-  // estimate of ||A|| and cond(A)
-  s.normA2 = s.normA2 + s.beta * s.beta;
-  s.normA = sqrt(s.normA2);
-  s.normA2 = s.normA2 + s.alpha * s.alpha;
-  s.maxrbar = s.maxrbar > rhobarold ? s.maxrbar : rhobarold;
-  if (s.iter > 1) s.minrbar = s.minrbar < rhobarold ? s.minrbar : rhobarold;
-  const double mx = s.maxrbar > rhotemp ? s.maxrbar : rhotemp;
-  const double mn = s.minrbar < rhotemp ? s.minrbar : rhotemp;
-  s.condA = mx / mn;
-  s.normAr = fabs(s.zetabar);
-}
-
-// Initial values of src/utils/lsmr.jl:68-100 given alpha, beta.
-__device__ static void lsmr_init(Inst& s, int init_mode) {
-  s.zetabar = s.alpha * s.beta;
-  s.alphabar = s.alpha;
-  s.rho = 1.0;
-  s.rhobar = 1.0;
-  s.cbar = 1.0;
-  s.sbar = 0.0;
-  s.betadd = s.beta;
-  s.betad = 0.0;
-  s.rhodold = 1.0;
-  s.tautildeold = 0.0;
-  s.thetatilde = 0.0;
-  s.zeta = 0.0;
-  s.d = 0.0;
-  s.normA = -1.0;
-  s.condA = -1.0;
-  s.normx = -1.0;
-  s.normA2 = s.alpha * s.alpha;
-  s.maxrbar = 0.0;
-  s.minrbar = 1e100;
-  s.normb = s.beta;
-  s.istop = 0;
-  s.normr = s.beta;
-  s.normAr = s.alpha * s.beta;
-  s.iter = 0;
-  s.pending = 0;
-  s.upd_mode = init_mode;  // h <- v, hbar <- 0 (and x <- 0) at the next reduce
-  s.do_v = 1;
-  s.active = (s.normAr != 0.0 && s.maxiter > 0 && !s.skip_lsmr) ? 1 : 0;
-  // a NaN or infinite right-hand side: the reference runs maxiter iterations
-  // on NaN norms (no test can pass) and reports istop = 7, not converged;
-  // here the instance stops at once with the same verdict
-  if (!isfinite(s.normAr)) {
-    s.active = 0;
-    s.istop = 7;
-  }
-  s.ex_av = s.s_v;
-  s.ex_au = -s.alpha * s.u_scale;
-  if (!s.active) deactivate(s);
-}
 
 __global__ void __launch_bounds__(kScalarThreads) k_scalar(ScalarArgs a) {
   __shared__ double red[3][kScalarThreads];

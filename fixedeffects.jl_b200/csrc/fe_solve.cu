@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 
+#include "fe_coef.h"
 #include "fe_plan.h"
 #include "fe_solve.h"
 
@@ -145,7 +146,9 @@ int solve(fe_plan* pl, const SolveReq& rq) {
     const int nc = (int)std::min<int64_t>(C, ncols - col0);
     int st;
     if (rq.before_tile && (st = rq.before_tile(rq.hook_ctx, col0, nc))) return st;
-    switch (C) {
+    int done = 0;
+    if (coef_takes(pl, rq, C) && (st = coef_solve_tile(pl, rq, C, col0, nc, res, &done))) return st;
+    if (!done) switch (C) {
       case 1: st = solve_tile_C<1>(pl, rq, col0, nc, res); break;
       case 2: st = solve_tile_C<2>(pl, rq, col0, nc, res); break;
       case 4: st = solve_tile_C<4>(pl, rq, col0, nc, res); break;
@@ -153,7 +156,7 @@ int solve(fe_plan* pl, const SolveReq& rq) {
       case 16: st = solve_tile_C<16>(pl, rq, col0, nc, res); break;
       default: st = solve_tile_C<32>(pl, rq, col0, nc, res); break;
     }
-    if (st) return st;
+    if (!done && st) return st;
     if (rq.after_tile && (st = rq.after_tile(rq.hook_ctx, col0, nc))) return st;
     // per-column verdicts: a column's instances are (problem p, column j);
     // with several problems the column aggregates them (max iterations, all

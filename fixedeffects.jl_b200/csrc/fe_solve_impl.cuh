@@ -28,6 +28,7 @@
 #include "fe_exdm_pipe.cuh"
 #include "fe_kernels.cuh"
 #include "fe_plan.h"
+#include "fe_prof.h"
 #include "fe_solve.h"
 
 namespace fe {
@@ -160,39 +161,6 @@ __global__ void k_coefs(const TX* __restrict__ X, int C, int j, int64_t base, in
 }
 
 static inline unsigned grid1(int64_t n, int b = 256) { return (unsigned)((n + b - 1) / b); }
-
-// ---------------------------------------------------------------------------
-// profiling: CUDA events around launches on the plan's stream
-// ---------------------------------------------------------------------------
-struct ProfScope {
-  fe_plan* pl;
-  const char* name;
-  double bytes;
-  cudaEvent_t a = nullptr, b = nullptr;
-  ProfScope(fe_plan* p, const char* n, double by) : pl(p), name(n), bytes(by) {
-    if (!pl->prof.on) return;
-    a = take();
-    b = take();
-    cudaEventRecord(a, pl->stream);
-  }
-  cudaEvent_t take() {
-    if (!pl->prof.pool.empty()) {
-      cudaEvent_t e = pl->prof.pool.back();
-      pl->prof.pool.pop_back();
-      return e;
-    }
-    cudaEvent_t e;
-    cudaEventCreate(&e);
-    return e;
-  }
-  ~ProfScope() {
-    if (!pl->prof.on) return;
-    cudaEventRecord(b, pl->stream);
-    pl->prof.pending.push_back({name, {a, b}});
-    pl->prof.bytes_per_launch[name] = bytes;
-  }
-};
-
 
 // ---------------------------------------------------------------------------
 // solve context for one tile
