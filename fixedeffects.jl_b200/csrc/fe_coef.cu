@@ -3,6 +3,7 @@
 #include "fe_coef.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "fe_prof.h"
@@ -138,9 +139,7 @@ static int coef_weights(fe_plan* pl, int f, int mask, const double** out) {
 }
 
 // Work items: consecutive levels packed into windows, longer levels cut into
-// pieces.  A warp has 32 / (CL << rlog) teams; rlog is the smallest with which
-// a round of levels of mean length fits a window, and an item holds whole
-// rounds, so that no team idles for want of a level.  Levels longer than a
+// pieces.  A warp has 32 / (CL << rlog) teams that take a level each.  Levels longer than a
 // quarter of a warp's share of the positions are cut, so that few long levels
 // still fill the GPU evenly (but not below 4 steps of a warp: a level of
 // several pieces costs a handshake and a norm slot).
@@ -164,11 +163,25 @@ static int coef_items(fe_plan* pl, int C, int window, CoefPlan::Items** out) {
     const std::vector<int64_t>& off = pl->seg_off[k];
     const int64_t nl = pl->nlev[k];
     const double avg = nl > 0 ? std::max(1.0, (double)pl->seg_len[k] / (double)nl) : 1.0;
-    int rlog = 0;
-    while ((cl << rlog) < 32 && avg * (32 / (cl << rlog)) > window) ++rlog;
-    const int nt = 32 / (cl << rlog);
-    const int rounds = std::max(1, (int)(window / (avg * nt)));
-    const int cap = std::min(32, nt * rounds);
+    // the cheapest team size by the passes' instruction counts: a window, a
+    // round of its teams, a step of a round (a level is about two standard
+    // deviations longer than the mean where it decides the round's length)
+    const int fit = std::max(1, std::min(32, (int)(window / avg)));
+    int rlog = 0, cap = fit;
+    double best = 1e300;
+    for (int r = 0; (cl << r) <= 32; ++r) {
+      const int nt = 32 / (cl << r);
+      const double steps = std::ceil((avg + 2.0 * std::sqrt(avg)) / (1 << r));
+      for (const int n : {fit, fit / nt * nt}) {
+        if (n < 1) continue;
+        const double cost = (150.0 + (n + nt - 1) / nt * (60.0 + 12.0 * r + 12.0 * steps)) / (n * avg);
+        if (cost < best) {
+          best = cost;
+          rlog = r;
+          cap = n;
+        }
+      }
+    }
     its->rlog[f] = rlog;
     if (f == cp.nf) its->multi_p = its->nmulti;
     its->piece0[f] = its->pieces;
@@ -437,7 +450,7 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
   }
   // small problems take few CTAs (a barrier costs the more the more arrive)
   const int64_t grid = std::max<int64_t>(
-      1, std::min<int64_t>((int64_t)its->occ * sms, (N * ((C + 3) / 4) + 511) / 512));
+      1, std::min<int64_t>((int64_t)its->occ * sms, (N * ((C + 3) / 4) + kCoefThreads - 1) / kCoefThreads));
   if ((st = cp.y.ensure((size_t)N * C * es))) return st;
   if ((st = cp.zb.ensure(pn * rc))) return st;
   if ((st = cp.z.ensure(pn * rc))) return st;

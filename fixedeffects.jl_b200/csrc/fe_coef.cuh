@@ -8,13 +8,14 @@
 // an iteration reads the level ids (and weights) once in every FE's order and
 // gathers one row of a coefficient table per entry, from L1 or L2 unless the
 // primary FE's table outgrows them, in two passes.  Large problems are bound
-// by the passes' instructions and the latency of their gathers (0.8 warp
-// instructions per SM and cycle, 5 per row), small ones by the two barriers
-// and the scalar step of an iteration (5 us of 27 at 800k rows).  Measured per
-// solve, before and after: 100M rows x 8 weighted columns 81.7 -> 39.1 ms,
-// 10M x 1 with three effects, one interacted, 3.42 -> 2.99 ms, 150k x 5
-// 0.90 -> 0.52 ms, 2k x 1 0.40 -> 0.16 ms, 800k x 1 of 5184 iterations
-// 315 -> 152 ms (FP64 throughout needs one inner solve where FP32 took three).
+// by the passes' instructions and the latency of their gathers (1.2 warp
+// instructions per SM and cycle, 4 to 5 per row), small ones by the chain of
+// loads of a pass, the two barriers and the scalar step of an iteration (10,
+// 9 and 4 us at 800k rows).  Measured per
+// solve, against the row-side loop: 100M rows x 8 weighted columns 81.7 ->
+// 38.7 ms, 10M x 1 with three effects, one interacted, 3.7 -> 3.0 ms, 150k x 5
+// 0.91 -> 0.40 ms, 2k x 1 0.46 -> 0.15 ms, 800k x 1 of 5184 iterations 274 ->
+// 121 ms (FP64 throughout needs one inner solve where FP32 took three).
 #pragma once
 
 #include <algorithm>
@@ -38,10 +39,14 @@ struct CoefShape {
   static constexpr int CL = C / VEC;
   static constexpr int R = 32 / CL;
 };
-// resident CTAs per SM: 32 warps of up to 64 registers, or 16 of up to 128
+// resident CTAs per SM: 16 warps of up to 128 registers, which keeps the walk
+// free of spills (at 64 registers their reloads took half of L1's cycles), or
+// 32 warps of 64 where the passes wait for the gathers of a large table.
+// Measured, pair of passes: 800k x 1 28 us with 32 warps, 19 us with 16; 2M x
+// 3 weighted 106 and 95 us; 100M x 8 weighted 3.39 and 3.49 ms.
 template <int C, int NG, int W>
 constexpr int kCoefCtas() {
-  return C <= 8 && NG <= 2 && W <= 1 ? 2 : 1;
+  return C == 8 && NG == 1 && W < 2 ? 2 : 1;
 }
 // rows in flight per lane of a pass with G gathers per row
 template <int C, int NG, int W>
@@ -191,7 +196,8 @@ __device__ __forceinline__ void coef_totals(CoefSmem<C>& sm, const CoefArgs& a, 
     const int col = threadIdx.x / 16, w = threadIdx.x % 16;
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
-      double s = col < C ? sm.red[k][w][col] : 0.0;
+      double s = 0.0;
+      for (int q = w; q < kCoefWarps && col < C; q += 16) s += sm.red[k][q][col];
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (w == 0 && col < C) sm.tot[k][col] = s;
@@ -249,14 +255,25 @@ __device__ __forceinline__ void coef_sweep(const CoefArgs& a, const CoefSide& sd
   auto begin_of = [&](const int4& d) -> uint32_t {  // the lane's level of a whole-level item
     return lane < d.w ? (uint32_t)__ldg(off + d.z + lane) : (uint32_t)d.y;
   };
+  const int32_t* ia[Row::kI > 0 ? Row::kI : 1];
+  const double* da[Row::kD > 0 ? Row::kD : 1];
+#pragma unroll
+  for (int i = 0; i < Row::kI; ++i) ia[i] = row.idx_array(i);
+#pragma unroll
+  for (int i = 0; i < Row::kD; ++i) da[i] = row.dbl_array(i);
   int4 cur = item(it), nxt = item(it + nw), nn = item(it + 2 * nw);
   uint32_t lb = begin_of(cur), lbn = begin_of(nxt);
+  // the single constant of the lane's level, ahead of its rows
+  auto ahead_of = [&](const int4& d) -> double {
+    return Epi::kAhead && lane < d.w ? __ldg(epi.lev + d.z + lane) : 0.0;
+  };
+  double ah = ahead_of(cur), ahn = ahead_of(nxt);
   auto issue = [&](uint32_t q0, uint32_t q1, int stage) {
     unsigned char* const st = ring + stage * kBytes;
     const uint32_t qa = q0 & ~3u, n = q1 - qa, left = npos - qa;
 #pragma unroll
     for (int i = 0; i < Row::kI; ++i) {
-      const int32_t* const src = row.idx_array(i);
+      const int32_t* const src = ia[i];
       if (!src) continue;
       const uint32_t c = lane * 4;
       if (c < n)
@@ -264,7 +281,7 @@ __device__ __forceinline__ void coef_sweep(const CoefArgs& a, const CoefSide& sd
     }
 #pragma unroll
     for (int i = 0; i < Row::kD; ++i) {
-      const double* const src = row.dbl_array(i);
+      const double* const src = da[i];
       if (!src) continue;
 #pragma unroll
       for (int h = 0; h < P; h += 64) {
@@ -316,7 +333,9 @@ __device__ __forceinline__ void coef_sweep(const CoefArgs& a, const CoefSide& sd
         const uint32_t b = __shfl_sync(kAll, lb, i & 31) - qa;
         const uint32_t e = __shfl_sync(kAll, le, i & 31) - qa;
         const bool own = i < cur.w;
-        const typename Epi::Pre pre = epi.pre(own ? cur.z + i : -1);
+        typename Epi::Pre pre;
+        if constexpr (Epi::kAhead) pre.v[0] = __shfl_sync(kAll, ah, i & 31);
+        else pre = epi.pre(own ? cur.z + i : -1);
         acc.zero();
         walk(b + rr, own ? e : 0, 1u << rlog);
         __syncwarp();
@@ -386,6 +405,8 @@ __device__ __forceinline__ void coef_sweep(const CoefArgs& a, const CoefSide& sd
       nxt = nn;
       nn = item(it + 2 * nw);
       lbn = begin_of(nxt);
+      ah = ahn;
+      ahn = ahead_of(nxt);
     }
     q0 = n0;
     q1 = n1;
@@ -765,6 +786,7 @@ __device__ __forceinline__ void coef_clear(double (&n)[NQ][CoefShape<C>::VEC]) {
 // an epilogue of coef_sweep: NL constants per level, loaded ahead, and the body
 template <int NL, class Body>
 struct CoefEpi {
+  static constexpr bool kAhead = NL == 1;
   const double* lev;
   Body body;
   struct Pre {
