@@ -54,23 +54,29 @@ static __global__ void k_lev_other(const double* __restrict__ scale,
   lev[4 * l + 3] = 0.0;
 }
 
-static int coef_plan(fe_plan* pl) {
+// the other FEs and their table rows
+static CoefPlan& coef_layout(fe_plan* pl) {
   if (!pl->coef) pl->coef = std::make_shared<CoefPlan>();
   CoefPlan& cp = *pl->coef;
+  if (cp.laid_out) return cp;
+  for (int k = 0; k < pl->K; ++k)
+    if (k != pl->primary) {
+      cp.fe[cp.nf] = k;
+      cp.base[cp.nf] = cp.rows;
+      cp.rows += pl->nlev[k];
+      ++cp.nf;
+    }
+  cp.laid_out = true;
+  return cp;
+}
+
+static int coef_plan(fe_plan* pl) {
+  CoefPlan& cp = coef_layout(pl);
   cudaStream_t s = pl->stream;
   const int kp = pl->primary;
   const int64_t N = pl->N;
   int st = 0;
   if (!cp.built) {
-    cp.nf = 0;
-    cp.rows = 0;
-    for (int k = 0; k < pl->K; ++k)
-      if (k != kp) {
-        cp.fe[cp.nf] = k;
-        cp.base[cp.nf] = cp.rows;
-        cp.rows += pl->nlev[k];
-        ++cp.nf;
-      }
     for (int f = 0; f < cp.nf; ++f) {
       const int32_t* perm = pl->dev.perm[cp.fe[f]];
       if ((st = cp.zi[f].ensure((size_t)N * 4))) return st;
@@ -141,8 +147,9 @@ static int coef_weights(fe_plan* pl, int f, int mask, const double** out) {
 // Work items: consecutive levels packed into windows, longer levels cut into
 // pieces.  A warp has 32 / (CL << rlog) teams that take a level each.  Levels longer than a
 // quarter of a warp's share of the positions are cut, so that few long levels
-// still fill the GPU evenly (but not below 4 steps of a warp: a level of
-// several pieces costs a handshake and a norm slot).
+// still fill the GPU evenly, but to no less than 1024 positions where the share
+// is more (a piece costs a handshake of about 1.5 us) and no less than 4 steps
+// of a warp.
 static int coef_items(fe_plan* pl, int C, int window, CoefPlan::Items** out) {
   CoefPlan& cp = *pl->coef;
   std::unique_ptr<CoefPlan::Items>& slot = cp.items[{C, window}];
@@ -155,7 +162,8 @@ static int coef_items(fe_plan* pl, int C, int window, CoefPlan::Items** out) {
   FE_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device));
   const int cl = C >= 4 ? C / 4 : 1;
   const int64_t share = pl->N / std::max<int64_t>(1, (int64_t)sms * kCoefWarps);
-  const int64_t psz = std::max<int64_t>(4 * (32 / cl), std::min<int64_t>(16384, share / 4));
+  const int64_t psz = std::max<int64_t>(
+      4 * (32 / cl), std::min<int64_t>(16384, std::min(share, std::max<int64_t>(1024, share / 4))));
   std::vector<CoefItem> whole, items;
   std::vector<CoefPiece> pcs;
   for (int f = 0; f <= cp.nf; ++f) {
@@ -396,13 +404,91 @@ bool coef_takes(const fe_plan* pl, const SolveReq& rq, int C) {
          pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0;
 }
 
-static const void* kernel_of(int C, int nf, int w, size_t* smem) {
+static const void* kernel_of(int C, int nf, int w, bool plain, size_t* smem) {
   switch (C) {
-    case 1: *smem = coef_smem_bytes<1>(nf, w); return coef_kernel<1>(nf, w);
-    case 2: *smem = coef_smem_bytes<2>(nf, w); return coef_kernel<2>(nf, w);
-    case 4: *smem = coef_smem_bytes<4>(nf, w); return coef_kernel<4>(nf, w);
-    default: *smem = coef_smem_bytes<8>(nf, w); return coef_kernel<8>(nf, w);
+    case 1:
+      *smem = coef_smem_bytes<1>(nf, w);
+      return plain ? plain_kernel<1>(nf, w) : coef_kernel<1>(nf, w);
+    case 2:
+      *smem = coef_smem_bytes<2>(nf, w);
+      return plain ? plain_kernel<2>(nf, w) : coef_kernel<2>(nf, w);
+    case 4:
+      *smem = coef_smem_bytes<4>(nf, w);
+      return plain ? plain_kernel<4>(nf, w) : coef_kernel<4>(nf, w);
+    default:
+      *smem = coef_smem_bytes<8>(nf, w);
+      return plain ? plain_kernel<8>(nf, w) : coef_kernel<8>(nf, w);
   }
+}
+
+// What both cooperative kernels of a tile need: work items, kernel, grid,
+// buffers of partial sums and the zeroed barrier.  *grid = 0: it does not fit.
+struct CoefLaunch {
+  CoefPlan::Items* its = nullptr;
+  const void* kern = nullptr;
+  size_t smem = 0;
+  int64_t grid = 0;
+  int weights = 0;
+};
+static int coef_prepare(fe_plan* pl, int C, bool plain, CoefLaunch* l, CoefArgs* a) {
+  CoefPlan& cp = *pl->coef;
+  const int nf = cp.nf;
+  l->weights = pl->weighted ? 1 : 0;
+  for (int k = 0; k < pl->K; ++k)
+    if (pl->interacted[k]) l->weights = 2;
+  int st = coef_items(pl, C, coef_window(nf, l->weights), &l->its);
+  if (st) return st;
+  CoefPlan::Items* its = l->its;
+  l->kern = kernel_of(C, nf, l->weights, plain, &l->smem);
+  int sms = 148;
+  FE_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device));
+  // opt-in shared memory, once per kernel and device
+  static PerDeviceOnce attr_set[2][4][9];
+  const int ci = C == 1 ? 0 : C == 2 ? 1 : C == 4 ? 2 : 3;
+  PerDeviceOnce& once = attr_set[plain][ci][(nf - 1) * 3 + l->weights];
+  if (once.needed(pl->device)) {
+    FE_CK(cudaFuncSetAttribute(l->kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l->smem));
+    once.done(pl->device);
+  }
+  if (!its->occ[plain] || its->occ_w[plain] != l->weights) {
+    int o = 0;
+    FE_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, l->kern, kCoefThreads, l->smem));
+    if (o < 1) return 0;
+    its->occ[plain] = o;
+    its->occ_w[plain] = l->weights;
+  }
+  // small problems take few CTAs (a barrier costs the more the more arrive)
+  const int64_t grid = std::max<int64_t>(
+      1, std::min<int64_t>((int64_t)its->occ[plain] * sms, (pl->N * ((C + 3) / 4) + 511) / 512));
+  const size_t rc = (size_t)C * 8;
+  if ((st = cp.part.ensure((size_t)2 * 3 * grid * rc))) return st;
+  if ((st = cp.ppart.ensure((size_t)std::max(its->pieces, 1) * rc))) return st;
+  if ((st = cp.mnrm.ensure((size_t)3 * std::max(its->nmulti, 1) * rc))) return st;
+  if ((st = cp.bar.ensure(64 + (size_t)C * sizeof(Inst)))) return st;
+  a->part = cp.part.as<double>();
+  a->ppart = cp.ppart.as<double>();
+  a->mnrm = cp.mnrm.as<double>();
+  a->nmulti = its->nmulti;
+  a->multi_p = its->multi_p;
+  a->pcnt = its->cnt.as<int32_t>();
+  a->bar = cp.bar.as<uint32_t>();
+  for (int f = 0; f <= nf; ++f) {
+    CoefSide& sd = f < nf ? a->f[f] : a->p;
+    const int k = f < nf ? cp.fe[f] : pl->primary;
+    sd.off = pl->d_off[k].as<int32_t>();
+    sd.perm = pl->dev.perm[k];
+    sd.items = its->dev[f].as<CoefItem>();
+    sd.pieces = its->piece[f].as<CoefPiece>();
+    sd.nitems = (int32_t)its->n[f];
+    sd.piece0 = its->piece0[f];
+    sd.n = (int32_t)pl->nlev[k];
+    sd.rlog = its->rlog[f];
+    sd.npos = (uint32_t)pl->N;
+  }
+  FE_CK(cudaMemsetAsync(cp.bar.p, 0, 64, pl->stream));
+  FE_CK(cudaMemsetAsync(its->cnt.p, 0, its->cnt.bytes, pl->stream));
+  l->grid = grid;
+  return 0;
 }
 
 #define FE_COEF_C(C, CALL)          \
@@ -424,49 +510,15 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
   const int64_t N = pl->N;
   const size_t es = 4, rc = (size_t)C * 8;
   const size_t pn = (size_t)std::max<int64_t>(pl->nlev[kp], 1), rn = (size_t)std::max<int64_t>(cp.rows, 1);
-  int weights = pl->weighted ? 1 : 0;
-  for (int k = 0; k < pl->K; ++k)
-    if (pl->interacted[k]) weights = 2;
-  CoefPlan::Items* its = nullptr;
-  if ((st = coef_items(pl, C, coef_window(nf, weights), &its))) return st;
-  size_t smem = 0;
-  const void* kern = kernel_of(C, nf, weights, &smem);
-  int sms = 148;
-  FE_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device));
-  // opt-in shared memory, once per kernel and device
-  static PerDeviceOnce attr_set[4][9];
-  const int ci = C == 1 ? 0 : C == 2 ? 1 : C == 4 ? 2 : 3;
-  PerDeviceOnce& once = attr_set[ci][(nf - 1) * 3 + weights];
-  if (once.needed(pl->device)) {
-    FE_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    once.done(pl->device);
-  }
-  if (!its->occ || its->occ_w != weights) {
-    int o = 0;
-    FE_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, kCoefThreads, smem));
-    if (o < 1) return 0;
-    its->occ = o;
-    its->occ_w = weights;
-  }
-  // small problems take few CTAs (a barrier costs the more the more arrive)
-  const int64_t grid = std::max<int64_t>(
-      1, std::min<int64_t>((int64_t)its->occ * sms, (N * ((C + 3) / 4) + kCoefThreads - 1) / kCoefThreads));
   if ((st = cp.y.ensure((size_t)N * C * es))) return st;
   if ((st = cp.zb.ensure(pn * rc))) return st;
   if ((st = cp.z.ensure(pn * rc))) return st;
   for (DevBuf* b : {&cp.ta, &cp.tb, &cp.h, &cp.hb, &cp.xx, &cp.c})
     if ((st = b->ensure(rn * rc))) return st;
-  if ((st = cp.part.ensure((size_t)2 * 3 * grid * rc))) return st;
-  if ((st = cp.ppart.ensure((size_t)std::max(its->pieces, 1) * rc))) return st;
-  if ((st = cp.mnrm.ensure((size_t)3 * std::max(its->nmulti, 1) * rc))) return st;
-  if ((st = cp.bar.ensure(64 + (size_t)C * sizeof(Inst)))) return st;
   CoefArgs a;
   memset(&a, 0, sizeof(a));
   for (int f = 0; f <= nf; ++f) {
     CoefSide& sd = f < nf ? a.f[f] : a.p;
-    const int k = f < nf ? cp.fe[f] : kp;
-    sd.off = pl->d_off[k].as<int32_t>();
-    sd.perm = pl->dev.perm[k];
     // the weight arrays of this order, each distinct one staged once
     int nd = 0;
     const auto slot = [&](int mask, int32_t* out) -> int {
@@ -502,14 +554,10 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
       sd.base = cp.base[f];
     }
     sd.lev = cp.lev[f].as<double>();
-    sd.items = its->dev[f].as<CoefItem>();
-    sd.pieces = its->piece[f].as<CoefPiece>();
-    sd.nitems = (int32_t)its->n[f];
-    sd.piece0 = its->piece0[f];
-    sd.n = (int32_t)pl->nlev[k];
-    sd.rlog = its->rlog[f];
-    sd.npos = (uint32_t)N;
   }
+  CoefLaunch cl;
+  if ((st = coef_prepare(pl, C, false, &cl, &a))) return st;
+  if (!cl.grid) return 0;
   a.y = cp.y.as<float>();
   a.ncols = ncols;
   a.zb = cp.zb.as<double>();
@@ -520,13 +568,6 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
   a.hb = cp.hb.as<double>();
   a.x = cp.xx.as<double>();
   a.c = cp.c.as<double>();
-  a.part = cp.part.as<double>();
-  a.ppart = cp.ppart.as<double>();
-  a.mnrm = cp.mnrm.as<double>();
-  a.nmulti = its->nmulti;
-  a.multi_p = its->multi_p;
-  a.pcnt = its->cnt.as<int32_t>();
-  a.bar = cp.bar.as<uint32_t>();
   a.inst = reinterpret_cast<Inst*>(static_cast<char*>(cp.bar.p) + 64);
   a.tol = rq.tol;
   a.theta = pl->opt_inner_theta;
@@ -535,8 +576,6 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
   a.rho = pl->opt_inner_rho * 1e-6;
   a.maxiter = rq.maxiter - 1;
   a.max_rounds = pl->opt_max_rounds;
-  FE_CK(cudaMemsetAsync(cp.bar.p, 0, 64, pl->stream));
-  FE_CK(cudaMemsetAsync(its->cnt.p, 0, its->cnt.bytes, pl->stream));
   {
     ProfScope ps(pl, "load", (double)N * (ncols + C) * es);
     FE_COEF_C(C, (st = rows_in<W>(pl, rq, col0, ncols, cp.y.as<float>())));
@@ -545,8 +584,8 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
   {
     ProfScope ps(pl, "coef_solve", 0.0);
     void* params[] = {&a};
-    FE_CK(cudaLaunchCooperativeKernel(kern, dim3((unsigned)grid), dim3(kCoefThreads), params, smem,
-                                      pl->stream));
+    FE_CK(cudaLaunchCooperativeKernel(cl.kern, dim3((unsigned)cl.grid), dim3(kCoefThreads), params,
+                                      cl.smem, pl->stream));
   }
   CoefResid r;
   memset(&r, 0, sizeof(r));
@@ -592,6 +631,69 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
       (per + 9.0 * rn * rc) * (double)(iters + rounds) + (double)N * C * es * (1 + nf) + (double)N * rc * nf;
   *done = 1;
   return prof_flush(pl);
+}
+
+// ---------------------------------------------------------------------------
+// the plain FP64 loop
+// ---------------------------------------------------------------------------
+// One problem, two to four FEs, unless an option names a launched kernel of
+// the loop or asks for the launches' times.
+bool plain_takes(const fe_plan* pl, const SolveReq& rq, int C) {
+  return C <= kCoefMaxCols && rq.precision == 0 && pl->nprob == 1 && !pl->xchg && pl->N > 0 &&
+         pl->K >= 2 && pl->K - 1 <= kCoefMaxFE && pl->perm_identity[pl->primary] &&
+         pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0;
+}
+
+int plain_loop(fe_plan* pl, int C, Inst* inst, double* U, double* V, double* H, double* Hb,
+               double* X, int* done) {
+  NvtxRange nv("fe: LSMR loop");
+  *done = 0;
+  CoefPlan& cp = coef_layout(pl);
+  const int kp = pl->primary, nf = cp.nf;
+  PlainArgs a;
+  memset(&a, 0, sizeof(a));
+  CoefLaunch cl;
+  int st = coef_prepare(pl, C, true, &cl, &a.s);
+  if (st) return st;
+  if (!cl.grid) return 0;
+  if ((st = cp.vs.ensure((size_t)pl->P * C * 8))) return st;
+  if ((st = cp.sp.ensure((size_t)std::max<int64_t>(pl->nlev[kp], 1) * C * 8))) return st;
+  for (int f = 0; f <= nf; ++f) {
+    CoefSide& sd = f < nf ? a.s.f[f] : a.s.p;
+    const int k = f < nf ? cp.fe[f] : kp;
+    sd.lev = pl->d_scale_d[k].as<double>();
+    sd.base = pl->lev_base[k];
+    if (f < nf) {
+      sd.dw = pl->dev.cwp_d[k];
+      continue;
+    }
+    sd.d[0] = pl->dev.cw_d[kp];
+    for (int g = 0; g < nf; ++g) {
+      sd.gi[g] = pl->dev.refs[cp.fe[g]];
+      sd.gb[g] = pl->lev_base[cp.fe[g]];
+      sd.d[1 + g] = pl->dev.cw_d[cp.fe[g]];
+    }
+  }
+  a.s.inst = inst;
+  a.u = U;
+  a.v = V;
+  a.vs = cp.vs.as<double>();
+  a.h = H;
+  a.hb = Hb;
+  a.x = X;
+  a.sp = cp.sp.as<double>();
+  void* params[] = {&a};
+  FE_CK(cudaLaunchCooperativeKernel(cl.kern, dim3((unsigned)cl.grid), dim3(kCoefThreads), params,
+                                    cl.smem, pl->stream));
+  *done = 1;
+  return 0;
+}
+
+// whether the loop's waits all ended (read once the stream has been waited for)
+int plain_status(fe_plan* pl, uint32_t* status) {
+  FE_CK(cudaMemcpyAsync(status, static_cast<char*>(pl->coef->bar.p) + 8, 4, cudaMemcpyDeviceToHost,
+                        pl->stream));
+  return 0;
 }
 
 }  // namespace fe

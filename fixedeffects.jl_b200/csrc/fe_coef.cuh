@@ -230,7 +230,7 @@ __device__ __forceinline__ void coef_copy16(void* smem, const void* gmem, int by
 // nrm; those of a level finished by whichever warp came last go to the level's
 // own slot (coef_totals adds them in order).
 template <int C, int NG, int W, class Row, int NQ, class Epi>
-__device__ __forceinline__ void coef_sweep(const CoefArgs& a, const CoefSide& sd, const Row& row,
+__device__ __forceinline__ void coef_sweep(const CoefArgs& a, const CoefSide& sd, Row row,
                                            double (&nrm)[NQ][CoefShape<C>::VEC], const Epi& epi) {
   using Sh = CoefShape<C>;
   constexpr int CL = Sh::CL, VEC = Sh::VEC;
@@ -314,7 +314,7 @@ __device__ __forceinline__ void coef_sweep(const CoefArgs& a, const CoefSide& sd
 #pragma unroll
         for (int u = 0; u < U; ++u) row.template load<P>(si, i + u * stride, qa, val[u]);
 #pragma unroll
-        for (int u = 0; u < U; ++u) row.template add<P>(sw, i + u * stride, val[u], acc);
+        for (int u = 0; u < U; ++u) row.template add<P>(sw, i + u * stride, qa, val[u], acc);
       }
       if (i < e) {
 #pragma unroll
@@ -322,7 +322,7 @@ __device__ __forceinline__ void coef_sweep(const CoefArgs& a, const CoefSide& sd
           if (i + u * stride < e) row.template load<P>(si, i + u * stride, qa, val[u]);
 #pragma unroll
         for (int u = 0; u < U - 1; ++u)
-          if (i + u * stride < e) row.template add<P>(sw, i + u * stride, val[u], acc);
+          if (i + u * stride < e) row.template add<P>(sw, i + u * stride, qa, val[u], acc);
       }
     };
     if (cur.w >= 0) {
@@ -337,6 +337,7 @@ __device__ __forceinline__ void coef_sweep(const CoefArgs& a, const CoefSide& sd
         if constexpr (Epi::kAhead) pre.v[0] = __shfl_sync(kAll, ah, i & 31);
         else pre = epi.pre(own ? cur.z + i : -1);
         acc.zero();
+        row.level(own ? cur.z + i : -1);
         walk(b + rr, own ? e : 0, 1u << rlog);
         __syncwarp();
         for (int o = CL; o < tl; o <<= 1)
@@ -345,6 +346,7 @@ __device__ __forceinline__ void coef_sweep(const CoefArgs& a, const CoefSide& sd
         if (own && rr == 0) epi(cur.z + i, pre, acc, jl, nrm);
       }
     } else {
+      row.level(cur.z);
       walk(q0 - qa + lane / CL, q1 - qa, Sh::R);
       __syncwarp();
       if (!same) {
@@ -420,7 +422,7 @@ __device__ __forceinline__ void coef_sweep(const CoefArgs& a, const CoefSide& sd
 // staged; load gathers the rows of local position i, add sums them up.  W: 0
 // no weights, 1 weights alone (one array for every entry), 2 interactions: the
 // entries' products of weights and interactions, slot 0.. of the distinct
-// arrays or -1 for 1.
+// arrays or -1 for 1.  level announces the team's level before its rows.
 // ---------------------------------------------------------------------------
 template <int W, int P>
 __device__ __forceinline__ double coef_weight(const double* sw, int slot, uint32_t i) {
@@ -451,6 +453,7 @@ struct CoefRowP {
       slot[g] = s.slot_g[g];
     }
   }
+  __device__ __forceinline__ void level(int) {}
   __device__ __forceinline__ const int32_t* idx_array(int i) const { return sd.gi[i]; }
   __device__ __forceinline__ const double* dbl_array(int i) const { return sd.d[i]; }
   template <int P>
@@ -459,7 +462,7 @@ struct CoefRowP {
     for (int g = 0; g < NG; ++g) v.t[g].load(t[g] + (int64_t)si[g * P + i] * C);
   }
   template <int P>
-  __device__ __forceinline__ void add(const double* sw, uint32_t i, const Val& v,
+  __device__ __forceinline__ void add(const double* sw, uint32_t i, uint32_t, const Val& v,
                                       CoefRow<C>& acc) const {
     if constexpr (NG == 1) {
       const double c = coef_weight<W, P>(sw, slot[0], i);
@@ -506,6 +509,7 @@ struct CoefRowF {
       slot[g] = s.slot_g[g];
     }
   }
+  __device__ __forceinline__ void level(int) {}
   __device__ __forceinline__ const int32_t* idx_array(int i) const {
     return i == 0 ? sd.zi : sd.gi[i - 1];
   }
@@ -517,7 +521,7 @@ struct CoefRowF {
     for (int g = 0; g < NO; ++g) v.t[g].load(t[g] + (int64_t)si[(1 + g) * P + i] * C);
   }
   template <int P>
-  __device__ __forceinline__ void add(const double* sw, uint32_t i, const Val& v,
+  __device__ __forceinline__ void add(const double* sw, uint32_t i, uint32_t, const Val& v,
                                       CoefRow<C>& acc) const {
     const double cz = coef_weight<W, P>(sw, sz, i);
     double c[NA];
@@ -546,6 +550,7 @@ struct CoefRowYP {
   const CoefSide& sd;
   double (&nrm)[CoefShape<C>::VEC];
   using Val = CoefRow<C>;
+  __device__ __forceinline__ void level(int) {}
   __device__ __forceinline__ const int32_t* idx_array(int) const { return nullptr; }
   __device__ __forceinline__ const double* dbl_array(int i) const { return i ? sd.dwx : sd.dw; }
   template <int P>
@@ -553,7 +558,7 @@ struct CoefRowYP {
     v.load(y + (int64_t)(qa + i) * C);
   }
   template <int P>
-  __device__ __forceinline__ void add(const double* sw, uint32_t i, const Val& v,
+  __device__ __forceinline__ void add(const double* sw, uint32_t i, uint32_t, const Val& v,
                                       CoefRow<C>& acc) const {
     const double w = coef_weight<W, P>(sw, sd.dw ? 0 : -1, i);
     const double wx = W == 2 ? coef_weight<2, P>(sw, sd.dwx ? 1 : -1, i) : w;
@@ -574,6 +579,7 @@ struct CoefRowYF {
   struct Val {
     CoefRow<C> y, z;
   };
+  __device__ __forceinline__ void level(int) {}
   __device__ __forceinline__ const int32_t* idx_array(int i) const {
     return i == 0 ? sd.zi : sd.perm;
   }
@@ -586,7 +592,7 @@ struct CoefRowYF {
     v.z.load(zb + (int64_t)si[i] * C);
   }
   template <int P>
-  __device__ __forceinline__ void add(const double* sw, uint32_t i, const Val& v,
+  __device__ __forceinline__ void add(const double* sw, uint32_t i, uint32_t, const Val& v,
                                       CoefRow<C>& acc) const {
     if (W == 2) {  // c_z, then c_y = w x_k
       const double cz = coef_weight<2, P>(sw, sd.slot_w >= 0 ? 0 : -1, i);

@@ -30,7 +30,8 @@ constexpr int kCoefMaxFE = 3;  // non-primary FEs of a plan that takes this path
 // of indices per lane, or half where five weight arrays are staged (nf, w as
 // coef_kernel).  Measured on 10M rows in levels of 10, three effects, one
 // interacted: 124 positions 136 + 242 us a pair of passes, 92 positions 278 +
-// 299 us (fewer levels a window, idle teams).
+// 299 us (fewer levels a window, idle teams); windows as long as shared memory
+// allows (up to 768 positions) took 100M x 8 from 38.6 to 45.4 ms a solve.
 constexpr int coef_window(int nf, int w) { return w == 2 && nf == 3 ? 60 : 124; }
 
 // Work item of a warp, one 16-byte load: levels [level, level + levels) at
@@ -95,6 +96,17 @@ struct CoefArgs {
   int32_t max_rounds;
 };
 
+// The plain FP64 loop (fe_plain.cuh): the sides' items and scales (lev), index
+// and entry arrays (primary: gi, and d[0] = its entries, d[1 + g] those of the
+// gathered FEs; with weights alone d[0] = sqrt(w) for all; others: perm, dw);
+// base, gb: slab rows.
+struct PlainArgs {
+  CoefArgs s;
+  double* u;                 // [N][C] rows
+  double *v, *vs, *h, *hb, *x;  // [P][C]; vs: scale times v
+  double* sp;                // [primary levels][C]: A_p'u
+};
+
 // status word of a finished solve (bar[2])
 constexpr uint32_t kCoefFallback = 1;  // take the row-side path instead
 
@@ -102,7 +114,7 @@ constexpr uint32_t kCoefFallback = 1;  // take the row-side path instead
 // order, built on the first solve that takes it, weights again after
 // fe_plan_update_weights.
 struct CoefPlan {
-  bool built = false, weights_built = false;
+  bool laid_out = false, built = false, weights_built = false;
   int nf = 0;
   int fe[kCoefMaxFE] = {};       // non-primary FEs
   int64_t base[kCoefMaxFE] = {};  // first table row of each
@@ -122,9 +134,10 @@ struct CoefPlan {
     int32_t rlog[kCoefMaxFE + 1] = {}, piece0[kCoefMaxFE + 1] = {};
     int32_t pieces = 0, nmulti = 0, multi_p = 0;
     DevBuf dev[kCoefMaxFE + 1], piece[kCoefMaxFE + 1], cnt;
-    int occ = 0, occ_w = -1;  // resident CTAs per SM of the solve kernel with weights occ_w
+    int occ[2] = {}, occ_w[2] = {-1, -1};  // resident CTAs per SM of the kernels with weights occ_w
   };
   std::map<std::pair<int, int>, std::unique_ptr<Items>> items;
+  DevBuf vs, sp;  // plain loop
   DevBuf y, zb, z, ta, tb, h, hb, xx, c, part, ppart, mnrm, bar;
 };
 
@@ -135,9 +148,21 @@ bool coef_takes(const fe_plan* pl, const SolveReq& rq, int C);
 int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int ncols,
                     std::vector<Inst>& out, int* done);
 
-// the solve kernel of a tile width (fe_coef_c*.cu)
+// Whether a plain FP64 solve of C columns runs its loop in one kernel, and the
+// loop: the instances at `inst` (device) hold the state after the first
+// bidiagonalisation step, U the rows, V, H, Hb, X the [P][C] slabs.  *done = 0:
+// it does not fit, the caller launches the loop.  plain_status (ordered on the
+// plan's stream): not 0 if a wait of the loop gave up.
+bool plain_takes(const fe_plan* pl, const SolveReq& rq, int C);
+int plain_loop(fe_plan* pl, int C, Inst* inst, double* U, double* V, double* H, double* Hb,
+               double* X, int* done);
+int plain_status(fe_plan* pl, uint32_t* status);
+
+// the kernels of a tile width (fe_coef_c*.cu)
 template <int C>
 const void* coef_kernel(int nf, int w);  // w: 0 none, 1 weights, 2 interactions too
+template <int C>
+const void* plain_kernel(int nf, int w);
 template <int C>
 size_t coef_smem_bytes(int nf, int w);
 

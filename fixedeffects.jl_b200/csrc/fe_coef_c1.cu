@@ -1,7 +1,10 @@
-// fe_coef_c1.cu -- the coefficient-side solve of 1-column tiles.
+// fe_coef_c1.cu -- the cooperative solves of 1-column tiles: on the
+// coefficient side (fe_coef.cuh) and the plain FP64 loop (fe_plain.cuh).
 #include "fe_coef.cuh"
+#include "fe_plain.cuh"
 
 namespace fe {
 template const void* coef_kernel<1>(int, int);
+template const void* plain_kernel<1>(int, int);
 template size_t coef_smem_bytes<1>(int, int);
 }  // namespace fe

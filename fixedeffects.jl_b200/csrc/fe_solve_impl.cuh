@@ -25,6 +25,7 @@
 #include <vector>
 
 #pragma once
+#include "fe_coef.h"
 #include "fe_exdm_pipe.cuh"
 #include "fe_kernels.cuh"
 #include "fe_plan.h"
@@ -1631,10 +1632,23 @@ static int solve_plain_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int n
     if ((e = launch_pupdate<C>(c, ST, pe, c.part_a, c.part_b, "pupdate", by.pupdate))) return e;
     return launch_scalar_phase(c, PH_ALPHA, 0);
   };
-  c.d.active = c.counters + 2;
-  st = run_loop(pl, c, (int)sizeof(T), cap, nact, body, nullptr);
-  c.d.active = nullptr;
-  if (st) return st;
+  int in_kernel = 0;  // the loop in one cooperative kernel
+  uint32_t loop_status = 0;
+  if constexpr (std::is_same<T, double>::value) {
+    if (nact > 0 && plain_takes(pl, rq, C)) {
+      ProfScope ps(pl, "plain_loop", by.expand + by.segsum + by.pupdate);
+      if ((st = plain_loop(pl, C, c.inst, U, V, w.H.as<double>(), w.Hb.as<double>(), X, &in_kernel)))
+        return st;
+    }
+  }
+  if (!in_kernel) {
+    c.d.active = c.counters + 2;
+    st = run_loop(pl, c, (int)sizeof(T), cap, nact, body, nullptr);
+    c.d.active = nullptr;
+    if (st) return st;
+  } else if ((st = plain_status(pl, &loop_status))) {
+    return st;
+  }
   if (rq.residuals) {
     // r = b - A x (src/AbstractFixedEffectSolver.jl:62)
     if ((st = launch_expand<T, C>(c, TabOne<T, T, vec_of<T, C>()>{X},
@@ -1646,6 +1660,10 @@ static int solve_plain_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int n
   out.resize(h.size());
   FE_CK(cudaMemcpyAsync(out.data(), c.inst, h.size() * sizeof(Inst), cudaMemcpyDeviceToHost, c.s));
   FE_CK(cudaStreamSynchronize(c.s));
+  if (loop_status) {
+    set_error_cstr("a grid-wide wait of the LSMR loop gave up");
+    return 4;  // FE_ERR_TIMEOUT
+  }
   if (!rq.residuals && rq.coefs) {
     if ((st = download_coefs<T>(pl, c, X, rq))) return st;
   }

@@ -141,3 +141,40 @@ def test_zero_weights_and_maxiter(fe):
         assert not cv and it == 3
         feM.close()
     assert _rel(out[0], out[1].astype(np.float64)) < REL
+
+
+@pytest.mark.parametrize("kind", ["tiny", "edges", "long", "four", "interacted", "primary"])
+@pytest.mark.parametrize("weighted,cols", [(False, 1), (True, 1), (True, 3), (False, 8)])
+def test_plain_loop_in_one_kernel(fe, oracle, kind, weighted, cols):
+    # FP64 solves of narrow tiles: the loop in one cooperative kernel against
+    # the launched loop (the same recurrences over sums in another order, so
+    # equal counts and rounding-level differences, scaled by the few iterations
+    # of these well-conditioned problems) and the oracle
+    n, refs, nlev, inter, rng = _problem(kind)
+    w = rng.uniform(0.5, 1.5, n) if weighted else None
+    Y = np.asfortranarray(rng.standard_normal((n, cols)) + (refs[0] % 7)[:, None] * 0.4)
+    fes = [fe.FixedEffect.from_refs(r, m, a) for r, m, a in zip(refs, nlev, inter)]
+    out = []
+    for launched in (False, True):
+        feM = fe.AbstractFixedEffectSolver(fes, w, "CUDA", np.float64)
+        if launched:
+            feM.set_option(fe._lib.FE_OPT_EXPAND_VARIANT, 0)
+            feM.set_option(fe._lib.FE_OPT_SEGSUM_VARIANT, 0)
+        feM.set_option(fe._lib.FE_OPT_PROFILE, 1)
+        R, its, cv = feM.solve_residuals(Y.copy(order="F"), tol=1e-8)
+        assert ("plain_loop" in feM.kernel_stats()) != launched
+        feM.set_option(fe._lib.FE_OPT_PROFILE, 0)
+        R2, its2, _ = feM.solve_residuals(Y.copy(order="F"), tol=1e-8)
+        b, it_b, cv_b = feM.solve_coefficients(Y[:, 0], tol=1e-8)
+        feM.close()
+        assert cv.all() and cv_b and np.array_equal(R, R2) and np.array_equal(its, its2)
+        out.append((R, its, b, it_b))
+    (R, its, b, it_b), (R1, its1, b1, it_b1) = out
+    assert np.abs(its - its1).max() <= 1 and abs(it_b - it_b1) <= 1
+    for j in range(cols):
+        if its[j] == its1[j]:
+            assert _rel(R[:, j], R1[:, j]) < 1e-10
+    r_o, it_o, _ = oracle.solve_residuals(Y[:, 0], refs, nlev, inter, w, tol=1e-8)
+    assert abs(int(its[0]) - int(it_o)) <= 1 and _rel(R[:, 0], r_o) < REL
+    fit = [sum(x * (1.0 if a is None else a) for x, a in zip(c, inter)) for c in (b, b1)]
+    assert np.linalg.norm(fit[0] - fit[1]) < REL * np.linalg.norm(fit[1])
