@@ -523,9 +523,7 @@ int plan_build_device(fe_plan* pl, const int64_t* const* refs, const int64_t* n_
       return 1;
     }
   }
-  FE_CK(cudaFree(d_r64.p));  // the raw refs are no longer needed
-  d_r64.p = nullptr;
-  d_r64.bytes = 0;
+  d_r64.release();  // the raw refs are no longer needed
 
   // observation order: stable sort by (problem, primary level)
   st = pl->d_obs_src.ensure((size_t)std::max<int64_t>(N, 1) * 4);

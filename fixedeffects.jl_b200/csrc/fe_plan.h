@@ -80,7 +80,17 @@ struct NvtxRange {
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  int pool_dev = -1;  // device whose pool p comes from, or -1
+  DevBuf() = default;
+  DevBuf(const DevBuf&) = delete;
+  DevBuf& operator=(const DevBuf&) = delete;
+  DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes), pool_dev(o.pool_dev) {
+    o.p = nullptr;
+    o.bytes = 0;
+    o.pool_dev = -1;
+  }
   ~DevBuf();
+  void release();
   int ensure(size_t n);  // grows (contents not preserved)
   template <typename T> T* as() const { return static_cast<T*>(p); }
 };
