@@ -390,18 +390,39 @@ static int rows_out(fe_plan* pl, const SolveReq& rq, int64_t col0, int ncols, fl
 // ---------------------------------------------------------------------------
 // driver
 // ---------------------------------------------------------------------------
+// Whether the passes' gathers pay: every further FE adds a gather per position
+// to every other FE's pass, so their cost grows with the square of the FEs'
+// number, while the row-side loop's grows with it.  Measured, solve of the
+// row-side loop / of this one:
+//   two FEs: 10M x 1 1.78 (100k x 100 levels) and 1.04 (2M x 200k), 100M x 8 2.2
+//   three: 1M x 1 1.80, 3M x 1 1.22 and, one interacted, 1.01; 3M x 2 1.17;
+//     10M x 4 and x 8 1.02 to 1.21; 10M x 1 1.12 where the others' levels fit
+//     L1 (100 and 1000), 0.88 where they do not (200k)
+//   four: 300k x 8 1.58, 1M x 1 1.52; one interacted: 300k x 1 1.46, 1M x 1
+//     1.02, 3M x 1 0.61
+static bool coef_pays(const fe_plan* pl, int C) {
+  const int nf = pl->K - 1;
+  if (nf == 1) return true;
+  if (nf == 2)
+    return C > 2 || pl->N <= 4'000'000 || pl->P - pl->nlev[pl->primary] - pl->K <= 16'384;
+  bool inter = false;
+  for (int k = 0; k < pl->K; ++k) inter = inter || pl->interacted[k];
+  return pl->N * C <= (inter ? 1'000'000 : 2'500'000);
+}
+
 // Mixed-precision residual solves of FP32 columns on plans whose primary FE is
 // absorbed, with at most kCoefMaxFE other FEs, unless an option names a kernel
 // of the row-side loop.  (FP64 columns keep the row-side iteration: theirs are
 // returned unrounded, so another iteration would show in them at the level of
-// the tolerance.  Every further FE adds a gather per position to every other
-// FE's pass, so the passes grow with the square of their number.)
+// the tolerance.  Tiles of 16 and 32 columns keep the row-side loop's FP32
+// rows: at 10M x 32, three FEs, an FP64 iteration here takes 2.5 ms against
+// 1.3 ms there.)
 bool coef_takes(const fe_plan* pl, const SolveReq& rq, int C) {
   return C <= kCoefMaxCols && rq.precision == 1 && rq.dtype == 1 && rq.residuals && pl->absorbable && pl->opt_absorb != 0 &&
          pl->opt_abs_scale != 0 && pl->nprob == 1 && !pl->xchg && pl->N > 0 &&
          pl->K - 1 <= kCoefMaxFE && pl->perm_identity[pl->primary] && pl->opt_exdm != 0 &&
          pl->opt_exdm_pipe < 0 && pl->opt_firm_atomic == 0 && pl->opt_fused_resid != 1 &&
-         pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0;
+         pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0 && coef_pays(pl, C);
 }
 
 static const void* kernel_of(int C, int nf, int w, bool plain, size_t* smem) {
@@ -457,9 +478,12 @@ static int coef_prepare(fe_plan* pl, int C, bool plain, CoefLaunch* l, CoefArgs*
     its->occ[plain] = o;
     its->occ_w[plain] = l->weights;
   }
-  // small problems take few CTAs (a barrier costs the more the more arrive)
-  const int64_t grid = std::max<int64_t>(
-      1, std::min<int64_t>((int64_t)its->occ[plain] * sms, (pl->N * ((C + 3) / 4) + 511) / 512));
+  // a CTA per 512 rows of up to 4 columns, one for the smallest problems, which
+  // then need no grid barrier (2k x 1: 148 us in one CTA, 159 in four; 20k x 1:
+  // 184 us at 512 rows a CTA, 210 at 2048)
+  const int64_t rows = pl->N * ((C + 3) / 4);
+  const int64_t grid =
+      rows <= 2048 ? 1 : std::min<int64_t>((int64_t)its->occ[plain] * sms, (rows + 511) / 512);
   const size_t rc = (size_t)C * 8;
   if ((st = cp.part.ensure((size_t)2 * 3 * grid * rc))) return st;
   if ((st = cp.ppart.ensure((size_t)std::max(its->pieces, 1) * rc))) return st;
@@ -636,10 +660,12 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
 // ---------------------------------------------------------------------------
 // the plain FP64 loop
 // ---------------------------------------------------------------------------
-// One problem, two to four FEs, unless an option names a launched kernel of
-// the loop or asks for the launches' times.
+// One problem of two to four FEs that is bound by launches, unless an option
+// names a launched kernel of the loop.  (Launched loop / this one: 200k x 1
+// 1.32, 1M x 1 1.17 to 1.22, 2M x 1 1.11, 4M x 1 0.96, 400k x 8 1.24, 1M x 8
+// 0.97; 10M x 1 in FEs of 2M, 200k and 20 levels 0.79.)
 bool plain_takes(const fe_plan* pl, const SolveReq& rq, int C) {
-  return C <= kCoefMaxCols && rq.precision == 0 && pl->nprob == 1 && !pl->xchg && pl->N > 0 &&
+  return pl->N * C <= 2'500'000 && C <= kCoefMaxCols && rq.precision == 0 && pl->nprob == 1 && !pl->xchg && pl->N > 0 &&
          pl->K >= 2 && pl->K - 1 <= kCoefMaxFE && pl->perm_identity[pl->primary] &&
          pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0;
 }

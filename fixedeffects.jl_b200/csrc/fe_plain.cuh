@@ -7,10 +7,10 @@
 //            lie in row order;
 //   levels:  the other FEs' sums over gathered rows of u, each followed at once
 //            by its level's update of v, h, hbar and x; the primary levels'.
-// Small problems are bound by the barriers and the scalar step, large ones by
-// the random 8-byte reads of u from L2.  Measured per solve, launched loop ->
-// this: 1M rows x 1, two effects, 0.68 -> 0.56 ms (the loop 0.53 -> 0.33), the
-// loop of 1M x 1 with three effects 0.86 -> 0.61 ms, 10M x 1 1.92 -> 1.89 ms.
+// Taken for small problems (plain_takes), which the barriers and the scalar
+// step bound; large ones are as fast launched.  Measured per solve, launched
+// loop -> this: 1M rows x 1, two effects, 0.68 -> 0.56 ms (the loop 0.53 ->
+// 0.33), the loop of 1M x 1 with three effects 0.86 -> 0.61 ms.
 #pragma once
 
 #include "fe_coef.cuh"
