@@ -51,7 +51,13 @@ extern "C" {
 #define FE_DTYPE_F64 0
 #define FE_DTYPE_F32 1
 
-/* plan options (fe_plan_set_option) */
+/* plan options (fe_plan_set_option).  Mixed-precision residual solves of FP32
+ * columns, in tiles of up to 8, run in one kernel on the coefficient side where
+ * that is measured to pay, and plain FP64 solves of small problems run their
+ * loop in one kernel; FE_OPT_EXPAND_VARIANT, _SEGSUM_VARIANT (both), _ABSORB = 0,
+ * _ABSORB_SCALE = 0, _FUSED_DEMEAN = 0, _EXDM_PIPE >= 0, _FIRM_ATOMIC != 0 and
+ * _FUSED_RESID = 1 (the first) name kernels of the launched loops and select
+ * those. */
 #define FE_OPT_TILE 1        /* column-tile width cap: 0 auto (<=32), 1,2,4,..,32 */
 #define FE_OPT_CHECK_EVERY 2 /* LSMR iterations between host convergence checks */
 #define FE_OPT_MAX_ROUNDS 3  /* FP64 refinement rounds (FE_PREC_MIXED) */
