@@ -410,6 +410,16 @@ static bool coef_pays(const fe_plan* pl, int C) {
   return pl->N * C <= (inter ? 1'000'000 : 2'500'000);
 }
 
+// Both cooperative kernels follow a row to its level in every FE, so every row
+// has to have one: an FE that the problem lacks (no levels, level ids 0) leaves
+// its rows outside the level order, on the slab's null row, which only the
+// launched loops hold.
+static bool every_row_has_levels(const fe_plan* pl) {
+  for (int k = 0; k < pl->K; ++k)
+    if (pl->seg_len[k] != pl->N) return false;
+  return true;
+}
+
 // Mixed-precision residual solves of FP32 columns on plans whose primary FE is
 // absorbed, with at most kCoefMaxFE other FEs, unless an option names a kernel
 // of the row-side loop.  (FP64 columns keep the row-side iteration: theirs are
@@ -422,7 +432,8 @@ bool coef_takes(const fe_plan* pl, const SolveReq& rq, int C) {
          pl->opt_abs_scale != 0 && pl->nprob == 1 && !pl->xchg && pl->N > 0 &&
          pl->K - 1 <= kCoefMaxFE && pl->perm_identity[pl->primary] && pl->opt_exdm != 0 &&
          pl->opt_exdm_pipe < 0 && pl->opt_firm_atomic == 0 && pl->opt_fused_resid != 1 &&
-         pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0 && coef_pays(pl, C);
+         pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0 && every_row_has_levels(pl) &&
+         coef_pays(pl, C);
 }
 
 static const void* kernel_of(int C, int nf, int w, bool plain, size_t* smem) {
@@ -667,7 +678,7 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
 bool plain_takes(const fe_plan* pl, const SolveReq& rq, int C) {
   return pl->N * C <= 2'500'000 && C <= kCoefMaxCols && rq.precision == 0 && pl->nprob == 1 && !pl->xchg && pl->N > 0 &&
          pl->K >= 2 && pl->K - 1 <= kCoefMaxFE && pl->perm_identity[pl->primary] &&
-         pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0;
+         pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0 && every_row_has_levels(pl);
 }
 
 int plain_loop(fe_plan* pl, int C, Inst* inst, double* U, double* V, double* H, double* Hb,
