@@ -672,6 +672,7 @@ extern "C" int fe_group_keys(const int64_t* const* keys, int32_t n_keys, int64_t
       cudaStreamDestroy(s);
     }
   } guard{s};
+  StreamScope scope(&s);
   DevBuf a64, cur, nxt;
   int st = a64.ensure((size_t)n * 8);
   if (!st) st = cur.ensure((size_t)n * 4);

@@ -50,7 +50,11 @@ int create_common(fe_plan** out, int32_t nprob, const int64_t* n_obs, int32_t K,
   }
   pl->xchg = xchg;
   pl->xchg_ctx = xchg_ctx;
-  int st = fe::plan_build(pl, nprob, n_obs, K, refs, n_levels, interaction, weights, device);
+  int st = 0;
+  {
+    fe::StreamScope scope(&pl->stream);
+    st = fe::plan_build(pl, nprob, n_obs, K, refs, n_levels, interaction, weights, device);
+  }
   if (st) {
     fe::plan_destroy(pl);
     return st;
@@ -184,6 +188,7 @@ int solve_common(fe_plan* plan, void* Y, void* const* cols, int32_t dtype, int64
     return FE_ERR_INVALID;
   }
   if (ncols == 0) return FE_OK;
+  fe::StreamScope scope(&plan->stream);
   const size_t es = dtype == FE_DTYPE_F64 ? 8 : 4;
   fe::SolveReq rq;
   rq.dtype = dtype;
@@ -530,6 +535,7 @@ int fe_solve_coefficients(fe_plan* plan, const void* y, int32_t dtype, int32_t p
     set_error("cudaSetDevice failed");
     return FE_ERR_CUDA;
   }
+  fe::StreamScope scope(&plan->stream);
   const int64_t N = plan->N;
   const size_t es = dtype == FE_DTYPE_F64 ? 8 : 4;
   fe::SolveReq rq;

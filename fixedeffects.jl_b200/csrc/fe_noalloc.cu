@@ -210,5 +210,15 @@ extern "C" int fe_plan_scales_noalloc(fe_plan* plan, int32_t fe_index, double* s
     set_error_cstr("fe_plan_scales_noalloc: kernel launch failed");
     return FE_ERR_CUDA;
   }
+  // what the plan does next (new weights, its end) waits for the reads above
+  if (s != plan->stream) {
+    e = cudaEventRecord(plan->noalloc_order, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(plan->stream, plan->noalloc_order, 0);
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      set_error_cstr("fe_plan_scales_noalloc: ordering the plan's stream failed");
+      return FE_ERR_CUDA;
+    }
+  }
   return FE_OK;
 }

@@ -86,10 +86,23 @@ static const DevicePool* device_pool(int dev) {
   return dp.pool ? &dp : nullptr;
 }
 
+static thread_local const StreamScope* t_scope = nullptr;
+StreamScope::StreamScope(const cudaStream_t* s) : stream(s), outer(t_scope) { t_scope = this; }
+StreamScope::~StreamScope() { t_scope = outer; }
+
+void wait_stream(cudaStream_t s) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &c) == cudaSuccess && c == cudaStreamCaptureStatusNone)
+    cudaStreamSynchronize(s);
+  (void)cudaGetLastError();
+}
+
 DevBuf::~DevBuf() { release(); }
 
-// Like cudaFree, waits for the device's work first: a block may be handed to
-// any stream next.
+// A freed block may be handed to any stream next, so the work that uses it is
+// waited for first (StreamScope).  The block is given back even where that
+// stream cannot be waited for (it is being captured): a plan's calls end with
+// their work done, so nothing of the plan is in flight there.
 void DevBuf::release() {
   if (!p) return;
   if (pool_dev < 0) {
@@ -97,7 +110,8 @@ void DevBuf::release() {
   } else {
     const int cur = current_device();
     if (cur != pool_dev) cudaSetDevice(pool_dev);
-    if (cudaDeviceSynchronize() == cudaSuccess) cudaFreeAsync(p, g_pools[pool_dev].stream);
+    if (t_scope && *t_scope->stream) wait_stream(*t_scope->stream);
+    cudaFreeAsync(p, g_pools[pool_dev].stream);
     if (cur != pool_dev) cudaSetDevice(cur);
     (void)cudaGetLastError();
   }
@@ -138,7 +152,7 @@ int DevBuf::ensure(size_t n) {
     return 3;  // FE_ERR_ALLOC
   }
   cudaError_t e = cudaErrorMemoryAllocation;
-  if (n <= kPoolBlock) {
+  if (n <= kPoolBlock && t_scope) {
     const int dev = current_device();
     if (const DevicePool* dp = device_pool(dev)) {
       e = cudaMallocFromPoolAsync(&p, n, dp->pool, dp->stream);
@@ -438,6 +452,7 @@ int plan_build(fe_plan* pl, int32_t nprob, const int64_t* n_obs, int32_t K,
 // update_weights!: src/SolverCPU.jl:67-76, ext/CUDAExt.jl:112-121.
 int plan_update_weights(fe_plan* pl, const double* weights) {
   NvtxRange nv("fe: weights and preconditioner");
+  StreamScope scope(&pl->stream);
   const int64_t N = pl->N;
   const int K = pl->K;
   cudaStream_t s = pl->stream;
@@ -912,7 +927,9 @@ int plan_items(fe_plan* pl, int C, ItemSet** out) {
 int plan_destroy(fe_plan* pl) {
   if (!pl) return 0;
   cudaSetDevice(pl->device);
-  if (pl->stream) cudaStreamSynchronize(pl->stream);
+  const cudaStream_t stream = pl->stream;
+  StreamScope scope(&stream);
+  if (stream) wait_stream(stream);
   for (auto& e : pl->prof.pool) cudaEventDestroy(e);
   for (auto& pr : pl->prof.pending) {
     cudaEventDestroy(pr.second.first);
@@ -925,10 +942,9 @@ int plan_destroy(fe_plan* pl) {
   if (pl->ring_down) cudaFreeHost(pl->ring_down);
   for (auto& g : pl->graphs)
     if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
-  cudaStream_t s = pl->stream;
   bool own = pl->own_stream;
   delete pl;
-  if (own && s) cudaStreamDestroy(s);
+  if (own && stream) cudaStreamDestroy(stream);
   return 0;
 }
 

@@ -76,6 +76,27 @@ struct NvtxRange {
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// Waits for the work of a stream, unless the stream is being captured (waiting
+// for it then would end the capture with an error).
+void wait_stream(cudaStream_t s);
+
+// Entered by every call that allocates: the stream that the call's kernels use
+// (read when a block is freed, so a plan's stream may be created meanwhile).
+// A block goes back to the pool once this stream's work is done: only the
+// stream is waited for, since waiting for the device while another thread
+// captures a graph on it is an error that also ends that capture.  Work on
+// other streams (the copies of a host solve, the caller's stream of
+// fe_plan_scales_noalloc) is waited for, or ordered before the plan's stream,
+// where it is queued.
+struct StreamScope {
+  explicit StreamScope(const cudaStream_t* s);
+  ~StreamScope();
+  StreamScope(const StreamScope&) = delete;
+  StreamScope& operator=(const StreamScope&) = delete;
+  const cudaStream_t* stream;
+  const StreamScope* outer;
+};
+
 // A device allocation owned by the plan.
 struct DevBuf {
   void* p = nullptr;
