@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 
 #include "fe_prof.h"
@@ -295,7 +296,7 @@ __global__ void __launch_bounds__(256) k_rows_out(const float* __restrict__ B, i
                                                   const uint32_t* __restrict__ bar) {
   constexpr int R = kRowElems / C, PER = kRowElems / 256;
   __shared__ float tile[R][C + 1];
-  if (bar[2]) return;  // the caller takes the row-side path
+  if (bar[1] | bar[2]) return;  // the caller takes the row-side path
   const int64_t i0 = (int64_t)blockIdx.x * R;
   float v[PER];
 #pragma unroll
@@ -333,7 +334,7 @@ template <int C>
 __global__ void __launch_bounds__(256) k_rows_resid(const CoefResid a, float* __restrict__ B, int64_t N,
                                                     const uint32_t* __restrict__ bar) {
   constexpr int VEC = C >= 2 ? 2 : 1, CL = C / VEC;
-  if (bar[2]) return;
+  if (bar[1] | bar[2]) return;
   const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
   const int64_t q = e / CL;
   if (q >= N) return;
@@ -453,6 +454,15 @@ static const void* kernel_of(int C, int nf, int w, bool plain, size_t* smem) {
   }
 }
 
+// Polls of a grid barrier before a wait gives up: tens of seconds, or
+// FE_B200_SPIN_LIMIT (read on every launch, so that a test can let waits run
+// out; the solve then takes the launched loops).
+static uint32_t spin_limit() {
+  const char* v = getenv("FE_B200_SPIN_LIMIT");
+  const unsigned long n = v ? strtoul(v, nullptr, 10) : 0;
+  return n > 0 && n < (1ul << 25) ? (uint32_t)n : 1u << 25;
+}
+
 // What both cooperative kernels of a tile need: work items, kernel, grid,
 // buffers of partial sums and the zeroed barrier.  *grid = 0: it does not fit.
 struct CoefLaunch {
@@ -507,6 +517,7 @@ static int coef_prepare(fe_plan* pl, int C, bool plain, CoefLaunch* l, CoefArgs*
   a->multi_p = its->multi_p;
   a->pcnt = its->cnt.as<int32_t>();
   a->bar = cp.bar.as<uint32_t>();
+  a->spins = spin_limit();
   for (int f = 0; f <= nf; ++f) {
     CoefSide& sd = f < nf ? a->f[f] : a->p;
     const int k = f < nf ? cp.fe[f] : pl->primary;
@@ -645,7 +656,7 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
   FE_CK(cudaStreamSynchronize(pl->stream));
   uint32_t bar[3];
   memcpy(bar, res.data(), sizeof(bar));
-  if (bar[2]) return prof_flush(pl);
+  if (bar[1] | bar[2]) return prof_flush(pl);
   out.resize((size_t)C);
   memcpy(out.data(), res.data() + 64, (size_t)C * sizeof(Inst));
   // bytes of the solve kernel: per iteration (the longest column's) the index
@@ -728,7 +739,7 @@ int plain_loop(fe_plan* pl, int C, Inst* inst, double* U, double* V, double* H, 
 
 // whether the loop's waits all ended (read once the stream has been waited for)
 int plain_status(fe_plan* pl, uint32_t* status) {
-  FE_CK(cudaMemcpyAsync(status, static_cast<char*>(pl->coef->bar.p) + 8, 4, cudaMemcpyDeviceToHost,
+  FE_CK(cudaMemcpyAsync(status, pl->coef->bar.as<uint32_t>() + 1, 4, cudaMemcpyDeviceToHost,
                         pl->stream));
   return 0;
 }

@@ -109,7 +109,10 @@ __device__ __forceinline__ int coef_col(int jl, int i) {
 
 // Grid-wide barrier of the co-resident CTAs of a cooperative launch.  A wait
 // is bounded: a CTA that gives up sets bar[1], which ends every other wait.
-__device__ __forceinline__ bool coef_barrier(uint32_t* bar, uint32_t& gen, int* sm_ok) {
+// (It may be seen by that CTA alone, the last one may have arrived since, so
+// bar[1] decides whether the launch counts, not what one CTA saw.)
+__device__ __forceinline__ bool coef_barrier(const CoefArgs& a, uint32_t& gen, int* sm_ok) {
+  uint32_t* const bar = a.bar;
   __syncthreads();
   if (gridDim.x == 1) return true;
   if (threadIdx.x == 0) {
@@ -119,7 +122,7 @@ __device__ __forceinline__ bool coef_barrier(uint32_t* bar, uint32_t& gen, int* 
     int ok = 1;
     uint32_t spins = 0;
     while ((int32_t)(*(volatile uint32_t*)bar - gen) < 0) {
-      if (++spins > (1u << 25) || ((spins & 255u) == 0 && *(volatile uint32_t*)(bar + 1) != 0)) {
+      if (++spins > a.spins || ((spins & 255u) == 0 && *(volatile uint32_t*)(bar + 1) != 0)) {
         atomicExch(bar + 1, 1u);
         ok = 0;
         break;
@@ -1040,7 +1043,7 @@ __global__ void __launch_bounds__(kCoefThreads, kCoefCtas<C, NG, W>()) k_coef(co
   double* tp = a.tb;
   double nr2 = 0.0;  // thread j < C: ||M b_j||^2
   coef_pass_yp<C, NG, W>(a, sm, par);
-  bool alive = coef_barrier(a.bar, gen, &sm.ok);
+  bool alive = coef_barrier(a, gen, &sm.ok);
   if (alive) {
     coef_totals<C, 2>(sm, a, par, a.multi_p, a.nmulti);
     par ^= 1;
@@ -1049,7 +1052,7 @@ __global__ void __launch_bounds__(kCoefThreads, kCoefCtas<C, NG, W>()) k_coef(co
       sm.nall[tid] = sm.tot[1][tid];
     }
     coef_pass_yf<C, NG, W>(a, sm, t, par);
-    alive = coef_barrier(a.bar, gen, &sm.ok);
+    alive = coef_barrier(a, gen, &sm.ok);
     if (alive) coef_totals<C, 2>(sm, a, par, 0, a.multi_p);
   }
   bool have_z = false;
@@ -1083,7 +1086,7 @@ __global__ void __launch_bounds__(kCoefThreads, kCoefCtas<C, NG, W>()) k_coef(co
         for (int i = 0; i < CoefShape<C>::VEC; ++i) nrm[1][i] += d * v.v[i] * v.v[i];
       }
       coef_publish<C, 2>(nrm, sm, a.part, par);
-      alive = coef_barrier(a.bar, gen, &sm.ok);
+      alive = coef_barrier(a, gen, &sm.ok);
       if (!alive) break;
       coef_totals<C, 2>(sm, a, par, 0, 0);
       par ^= 1;
@@ -1093,7 +1096,7 @@ __global__ void __launch_bounds__(kCoefThreads, kCoefCtas<C, NG, W>()) k_coef(co
     // inner LSMR
     while (any) {
       coef_pass_p<C, NG, W>(a, sm, t, par);
-      alive = coef_barrier(a.bar, gen, &sm.ok);
+      alive = coef_barrier(a, gen, &sm.ok);
       if (!alive) break;
       coef_totals<C, 1>(sm, a, par, a.multi_p, a.nmulti);
       par ^= 1;
@@ -1103,7 +1106,7 @@ __global__ void __launch_bounds__(kCoefThreads, kCoefCtas<C, NG, W>()) k_coef(co
       }
       __syncthreads();
       coef_pass_f<C, NG, W>(a, sm, t, tp, par);
-      alive = coef_barrier(a.bar, gen, &sm.ok);
+      alive = coef_barrier(a, gen, &sm.ok);
       if (!alive) break;
       coef_totals<C, NG == 1 ? 2 : 1>(sm, a, par, 0, a.multi_p);
       par ^= 1;
@@ -1116,22 +1119,22 @@ __global__ void __launch_bounds__(kCoefThreads, kCoefCtas<C, NG, W>()) k_coef(co
     if (!alive) break;
     if (__syncthreads_or(tid < C && sm.mode[tid] == 2)) {
       coef_pass_x<C, NG>(a, sm);
-      alive = coef_barrier(a.bar, gen, &sm.ok);
+      alive = coef_barrier(a, gen, &sm.ok);
       if (!alive) break;
     }
     coef_pass_p<C, NG, W>(a, sm, a.x, par);
     have_z = true;
     if (!outer) break;  // every column stopped at once: z of x = 0
-    alive = coef_barrier(a.bar, gen, &sm.ok);
+    alive = coef_barrier(a, gen, &sm.ok);
     if (!alive) break;
     par ^= 1;
     coef_pass_g<C, NG, W>(a, sm, t, par);
-    alive = coef_barrier(a.bar, gen, &sm.ok);
+    alive = coef_barrier(a, gen, &sm.ok);
     if (alive) coef_totals<C, 3>(sm, a, par, 0, a.multi_p);
   }
   if (blockIdx.x == 0) {
     if (tid < C) a.inst[tid] = sm.inst[tid];
-    if (tid == 0 && (sm.status || !alive)) a.bar[2] = kCoefFallback;
+    if (tid == 0 && sm.status) a.bar[2] = kCoefFallback;
   }
 }
 

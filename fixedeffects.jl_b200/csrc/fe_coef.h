@@ -90,6 +90,7 @@ struct CoefArgs {
   int32_t nmulti, multi_p;   // such levels; the primary FE's start at multi_p
   int32_t* pcnt;
   uint32_t* bar;             // [0] arrivals, [1] a wait gave up, [2] status
+  uint32_t spins;            // polls of a grid barrier before a wait gives up
   Inst* inst;
   double tol, theta, rho;
   int64_t maxiter;
@@ -107,7 +108,7 @@ struct PlainArgs {
   double* sp;                // [primary levels][C]: A_p'u
 };
 
-// status word of a finished solve (bar[2])
+// status word of a solve that came to its end (bar[1] == 0): bar[2]
 constexpr uint32_t kCoefFallback = 1;  // take the row-side path instead
 
 // Per-plan data of the path: index and weight arrays in every FE's level

@@ -204,11 +204,11 @@ __global__ void __launch_bounds__(kCoefThreads, 1) k_plain(const PlainArgs args)
       }
     }
   }
-  bool alive = coef_barrier(a.s.bar, gen, &sm.ok);
+  bool alive = coef_barrier(a.s, gen, &sm.ok);
   bool any = __syncthreads_or(tid < C && sm.inst[tid].active);
   while (alive && any) {
     plain_pass_u<C, NG, W>(a, sm, par);
-    alive = coef_barrier(a.s.bar, gen, &sm.ok);
+    alive = coef_barrier(a.s, gen, &sm.ok);
     if (!alive) break;
     coef_totals<C, 1>(sm, a.s, par, a.s.multi_p, a.s.nmulti);
     par ^= 1;
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kCoefThreads, 1) k_plain(const PlainArgs args)
     }
     __syncthreads();
     plain_pass_v<C, NG, W>(a, sm, par);
-    alive = coef_barrier(a.s.bar, gen, &sm.ok);
+    alive = coef_barrier(a.s, gen, &sm.ok);
     if (!alive) break;
     coef_totals<C, 2>(sm, a.s, par, 0, a.s.multi_p);
     par ^= 1;
@@ -257,10 +257,7 @@ __global__ void __launch_bounds__(kCoefThreads, 1) k_plain(const PlainArgs args)
     }
     any = __syncthreads_or(tid < C && sm.inst[tid].active);
   }
-  if (blockIdx.x == 0) {
-    if (tid < C) a.s.inst[tid] = sm.inst[tid];
-    if (tid == 0 && !alive) a.s.bar[2] = kCoefFallback;
-  }
+  if (blockIdx.x == 0 && tid < C) a.s.inst[tid] = sm.inst[tid];
 }
 
 template <int C>

@@ -1,0 +1,43 @@
+"""Bounded waits of the cooperative solves that run out (FE_B200_SPIN_LIMIT):
+whichever of the kernel's blocks give up, the call's result is that of the
+launched loops.  Nothing hangs: every wait ends by itself.
+
+The bar is the repository's 1e-6 on the residual's relative 2-norm.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+REL = 1e-6
+
+
+def _problem(fe, T, cols, n=60_013):
+    rng = np.random.default_rng(6)
+    refs, nlev = [rng.integers(1, m + 1, n) for m in (5000, 400, 9)], [5000, 400, 9]
+    Y = np.asfortranarray((rng.standard_normal((n, cols)) + (refs[1] % 5)[:, None]).astype(T))
+    feM = fe.AbstractFixedEffectSolver([fe.FixedEffect.from_refs(r, m) for r, m in zip(refs, nlev)],
+                                       None, "CUDA", T)
+    return feM, Y, refs, nlev
+
+
+def _rel(a, b):
+    return np.linalg.norm(a.astype(np.float64) - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("T", [np.float32])
+@pytest.mark.parametrize("limit", [1, 3, 10, 30, 100, 300])
+def test_result_does_not_depend_on_waits(fe, oracle, monkeypatch, T, limit):
+    feM, Y, refs, nlev = _problem(fe, T, 2)
+    R_o, _, _ = oracle.solve_residuals_cols(Y.astype(np.float64), refs, nlev, [None] * 3, None,
+                                            tol=1e-10)
+    monkeypatch.setenv("FE_B200_SPIN_LIMIT", str(limit))
+    for _ in range(4):
+        R, _, cv = feM.solve_residuals(Y.copy(order="F"), tol=1e-8)
+        assert cv.all() and max(_rel(R[:, j], R_o[:, j]) for j in range(2)) < REL
+        Z, _, cv = feM.solve_residuals(np.zeros_like(Y, order="F"), tol=1e-8)
+        assert cv.all() and not Z.any()
+    monkeypatch.delenv("FE_B200_SPIN_LIMIT")
+    R, _, cv = feM.solve_residuals(Y.copy(order="F"), tol=1e-8)
+    feM.close()
+    assert cv.all() and max(_rel(R[:, j], R_o[:, j]) for j in range(2)) < REL
