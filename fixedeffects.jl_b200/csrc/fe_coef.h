@@ -152,12 +152,13 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
 // Whether a plain FP64 solve of C columns runs its loop in one kernel, and the
 // loop: the instances at `inst` (device) hold the state after the first
 // bidiagonalisation step, U the rows, V, H, Hb, X the [P][C] slabs.  *done = 0:
-// it does not fit, the caller launches the loop.  plain_status (ordered on the
-// plan's stream): not 0 if a wait of the loop gave up.
+// it does not fit, the caller launches the loop.  plain_gave_up: device address
+// of a word that is not 0 after the loop's kernel if one of its waits gave up;
+// U, V, H, Hb and X are then unfinished.
 bool plain_takes(const fe_plan* pl, const SolveReq& rq, int C);
 int plain_loop(fe_plan* pl, int C, Inst* inst, double* U, double* V, double* H, double* Hb,
                double* X, int* done);
-int plain_status(fe_plan* pl, uint32_t* status);
+const uint32_t* plain_gave_up(const fe_plan* pl);
 
 // the kernels of a tile width (fe_coef_c*.cu)
 template <int C>

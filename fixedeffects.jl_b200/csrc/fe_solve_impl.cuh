@@ -123,9 +123,13 @@ __global__ void __launch_bounds__(256) k_unload(const double* __restrict__ Rw, i
                                                 int64_t col0, int ncols,
                                                 const int32_t* __restrict__ dst,
                                                 const double* __restrict__ sw,
-                                                TY* __restrict__ Y, int64_t N) {
+                                                TY* __restrict__ Y, int64_t N,
+                                                const uint32_t* __restrict__ gave_up) {
   constexpr int R = load_rows<C>();
   __shared__ double tile[R][C + load_pad<C>()];
+  // a loop in one kernel that did not come to its end: the columns stay the
+  // right-hand sides, the caller solves them again
+  if (gave_up && *gave_up) return;
   const int64_t i0 = (int64_t)blockIdx.x * R;
   double v[kLoadPer];
 #pragma unroll
@@ -1185,10 +1189,11 @@ static void launch_load(const fe_plan* pl, Ctx& c, const SolveReq& rq, int64_t c
       W ? pl->d_sw_orig.as<double>() : nullptr, pl->ws.B64.as<double>(), pl->N);
 }
 template <int C, typename TY, bool W>
-static void launch_unload(const fe_plan* pl, Ctx& c, const SolveReq& rq, int64_t col0, int ncols) {
+static void launch_unload(const fe_plan* pl, Ctx& c, const SolveReq& rq, int64_t col0, int ncols,
+                          const uint32_t* gave_up) {
   k_unload<TY, C, W><<<grid1(pl->N, load_rows<C>()), 256, 0, c.s>>>(
       pl->ws.R64.as<double>(), rq.ld, col0, ncols, pl->d_obs_dst.as<int32_t>(),
-      W ? pl->d_sw_orig.as<double>() : nullptr, (TY*)rq.Y, pl->N);
+      W ? pl->d_sw_orig.as<double>() : nullptr, (TY*)rq.Y, pl->N, gave_up);
 }
 
 template <int C>
@@ -1207,16 +1212,17 @@ static int load_tile(fe_plan* pl, Ctx& c, const SolveReq& rq, int64_t col0, int 
 }
 
 template <int C>
-static int unload_tile(fe_plan* pl, Ctx& c, const SolveReq& rq, int64_t col0, int ncols) {
+static int unload_tile(fe_plan* pl, Ctx& c, const SolveReq& rq, int64_t col0, int ncols,
+                       const uint32_t* gave_up = nullptr) {
   NvtxRange nv("fe: unload tile");
   if (pl->N == 0) return 0;
   ProfScope ps(pl, "unload", (double)pl->N * ncols * (rq.dtype == 0 ? 8 : 4) + (double)pl->N * C * 8);
   if (rq.dtype == 0)
-    pl->weighted ? launch_unload<C, double, true>(pl, c, rq, col0, ncols)
-                 : launch_unload<C, double, false>(pl, c, rq, col0, ncols);
+    pl->weighted ? launch_unload<C, double, true>(pl, c, rq, col0, ncols, gave_up)
+                 : launch_unload<C, double, false>(pl, c, rq, col0, ncols, gave_up);
   else
-    pl->weighted ? launch_unload<C, float, true>(pl, c, rq, col0, ncols)
-                 : launch_unload<C, float, false>(pl, c, rq, col0, ncols);
+    pl->weighted ? launch_unload<C, float, true>(pl, c, rq, col0, ncols, gave_up)
+                 : launch_unload<C, float, false>(pl, c, rq, col0, ncols, gave_up);
   FE_CK(cudaGetLastError());
   return 0;
 }
@@ -1563,7 +1569,7 @@ static int download_coefs(fe_plan* pl, Ctx& c, const TX* X, const SolveReq& rq) 
 // ---------------------------------------------------------------------------
 template <typename T, int C>
 static int solve_plain_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int ncols,
-                            std::vector<Inst>& out) {
+                            std::vector<Inst>& out, bool one_kernel = true) {
   NvtxRange nv("fe: tile (plain LSMR)");
   Ctx c;
   int st = prepare(pl, C, (int)sizeof(T), false, c);
@@ -1633,9 +1639,9 @@ static int solve_plain_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int n
     return launch_scalar_phase(c, PH_ALPHA, 0);
   };
   int in_kernel = 0;  // the loop in one cooperative kernel
-  uint32_t loop_status = 0;
+  uint32_t gave_up = 0;
   if constexpr (std::is_same<T, double>::value) {
-    if (nact > 0 && plain_takes(pl, rq, C)) {
+    if (one_kernel && nact > 0 && plain_takes(pl, rq, C)) {
       ProfScope ps(pl, "plain_loop", by.expand + by.segsum + by.pupdate);
       if ((st = plain_loop(pl, C, c.inst, U, V, w.H.as<double>(), w.Hb.as<double>(), X, &in_kernel)))
         return st;
@@ -1646,8 +1652,8 @@ static int solve_plain_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int n
     st = run_loop(pl, c, (int)sizeof(T), cap, nact, body, nullptr);
     c.d.active = nullptr;
     if (st) return st;
-  } else if ((st = plain_status(pl, &loop_status))) {
-    return st;
+  } else {
+    FE_CK(cudaMemcpyAsync(&gave_up, plain_gave_up(pl), 4, cudaMemcpyDeviceToHost, c.s));
   }
   if (rq.residuals) {
     // r = b - A x (src/AbstractFixedEffectSolver.jl:62)
@@ -1655,15 +1661,13 @@ static int solve_plain_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int n
                                   EpiBminusAx<double, T, vec_of<T, C>()>{B64, w.R64.as<double>(), nullptr, c.inst, 0},
                                   nullptr, "expand_final", by.expand)))
       return st;
-    if ((st = unload_tile<C>(pl, c, rq, col0, ncols))) return st;
+    if ((st = unload_tile<C>(pl, c, rq, col0, ncols, in_kernel ? plain_gave_up(pl) : nullptr)))
+      return st;
   }
   out.resize(h.size());
   FE_CK(cudaMemcpyAsync(out.data(), c.inst, h.size() * sizeof(Inst), cudaMemcpyDeviceToHost, c.s));
   FE_CK(cudaStreamSynchronize(c.s));
-  if (loop_status) {
-    set_error_cstr("a grid-wide wait of the LSMR loop gave up");
-    return 4;  // FE_ERR_TIMEOUT
-  }
+  if (gave_up) return solve_plain_tile<T, C>(pl, rq, col0, ncols, out, false);
   if (!rq.residuals && rq.coefs) {
     if ((st = download_coefs<T>(pl, c, X, rq))) return st;
   }

@@ -25,19 +25,24 @@ def _rel(a, b):
     return np.linalg.norm(a.astype(np.float64) - b) / np.linalg.norm(b)
 
 
-@pytest.mark.parametrize("T", [np.float32])
+@pytest.mark.parametrize("T", [np.float32, np.float64])
 @pytest.mark.parametrize("limit", [1, 3, 10, 30, 100, 300])
 def test_result_does_not_depend_on_waits(fe, oracle, monkeypatch, T, limit):
     feM, Y, refs, nlev = _problem(fe, T, 2)
     R_o, _, _ = oracle.solve_residuals_cols(Y.astype(np.float64), refs, nlev, [None] * 3, None,
                                             tol=1e-10)
     monkeypatch.setenv("FE_B200_SPIN_LIMIT", str(limit))
+    feM.set_option(fe._lib.FE_OPT_PROFILE, 1)
     for _ in range(4):
         R, _, cv = feM.solve_residuals(Y.copy(order="F"), tol=1e-8)
         assert cv.all() and max(_rel(R[:, j], R_o[:, j]) for j in range(2)) < REL
         Z, _, cv = feM.solve_residuals(np.zeros_like(Y, order="F"), tol=1e-8)
         assert cv.all() and not Z.any()
+    if limit == 1:  # no barrier is passed on the first poll by every block
+        stats = feM.kernel_stats()
+        assert ("demean64" if T == np.float32 else "expand") in stats
     monkeypatch.delenv("FE_B200_SPIN_LIMIT")
+    feM.set_option(fe._lib.FE_OPT_PROFILE, 0)
     R, _, cv = feM.solve_residuals(Y.copy(order="F"), tol=1e-8)
     feM.close()
     assert cv.all() and max(_rel(R[:, j], R_o[:, j]) for j in range(2)) < REL
