@@ -1,6 +1,8 @@
 // fe_lsmr.cuh -- the LSMR scalar recurrences of one instance, in FP64
 // (src/utils/lsmr.jl:46-222, lambda = 0), shared by the scalar kernel of the
-// row-side solves (fe_scalar.cu) and the coefficient-side solve (fe_coef.cuh).
+// row-side solves (fe_scalar.cu) and the one-kernel solves (fe_plain.cuh,
+// fe_coef.cuh).  Every multiply and add rounds separately, as in the
+// reference's scalar code, in whichever kernel they are compiled.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -8,6 +10,19 @@
 #include "fe_internal.h"
 
 namespace fe {
+
+// A double whose products and sums are rounded one by one (the compiler does
+// not contract them to fused multiply-adds).
+struct Rn {
+  double v;
+  __device__ __forceinline__ Rn(double x) : v(x) {}
+};
+__device__ __forceinline__ Rn operator*(Rn a, Rn b) { return __dmul_rn(a.v, b.v); }
+__device__ __forceinline__ Rn operator+(Rn a, Rn b) { return __dadd_rn(a.v, b.v); }
+__device__ __forceinline__ Rn operator-(Rn a, Rn b) { return __dadd_rn(a.v, -b.v); }
+__device__ __forceinline__ Rn operator-(Rn a) { return -a.v; }
+__device__ __forceinline__ Rn operator/(Rn a, Rn b) { return __ddiv_rn(a.v, b.v); }
+__device__ __forceinline__ Rn root(Rn a) { return __dsqrt_rn(a.v); }
 
 // Kernel coefficients of a stopped instance: the expand keeps U
 // (U <- 0*(A v) + 1*U) and the P-side update is skipped (upd_mode 0, no v).
@@ -21,11 +36,12 @@ __device__ static void deactivate(Inst& s) {
 
 __device__ static void lsmr_test(Inst& s) {
   // src/utils/lsmr.jl:188-215
-  const double test1 = s.normr / s.normb;
-  const double test2 = s.normAr / (s.normA * s.normr);
-  const double test3 = 1.0 / s.condA;
-  const double t1 = test1 / (1.0 + s.normA * s.normx / s.normb);
-  const double rtol = s.btol + s.atol * s.normA * s.normx / s.normb;
+  const Rn normA = s.normA, normr = s.normr, normAr = s.normAr, normb = s.normb, normx = s.normx;
+  const double test1 = (normr / normb).v;
+  const double test2 = (normAr / (normA * normr)).v;
+  const double test3 = (Rn(1.0) / s.condA).v;
+  const double t1 = (Rn(test1) / (Rn(1.0) + normA * normx / normb)).v;
+  const double rtol = (Rn(s.btol) + Rn(s.atol) * normA * normx / normb).v;
   int istop = 0;
   if (s.iter >= s.maxiter) istop = 7;
   else if (1.0 + test3 <= 1.0) istop = 6;
@@ -37,8 +53,9 @@ __device__ static void lsmr_test(Inst& s) {
   if (!istop && s.mode_inner) {
     // inner solve of the mixed mode: stop once the FP64 outer test is
     // expected to pass, or once normAr fell by inner_rho (the FP32 floor)
-    const double nAt = sqrt(s.normA2_prev + s.normA * s.normA);
-    if (s.normAr <= s.inner_theta_tol * nAt * s.normr || s.normAr <= s.inner_rho * s.normAr0)
+    const Rn nAt = root(Rn(s.normA2_prev) + normA * normA);
+    if (s.normAr <= (Rn(s.inner_theta_tol) * nAt * normr).v ||
+        s.normAr <= (Rn(s.inner_rho) * s.normAr0).v)
       istop = 2;
   }
   s.istop = istop;
@@ -46,54 +63,65 @@ __device__ static void lsmr_test(Inst& s) {
 
 __device__ static void lsmr_rotate(Inst& s) {
   // src/utils/lsmr.jl:113-186, lambda = 0
-  const double lambda = 0.0;
-  const double alphahat = sqrt(s.alphabar * s.alphabar + lambda * lambda);
-  const double chat = s.alphabar / alphahat;
-  const double shat = lambda / alphahat;
-  const double rhoold = s.rho;
-  s.rho = sqrt(alphahat * alphahat + s.beta * s.beta);
-  const double c = alphahat / s.rho;
-  const double sn = s.beta / s.rho;
-  const double thetanew = sn * s.alpha;
-  s.alphabar = c * s.alpha;
-  const double rhobarold = s.rhobar;
-  const double zetaold = s.zeta;
-  const double thetabar = s.sbar * s.rho;
-  const double rhotemp = s.cbar * s.rho;
-  s.rhobar = sqrt((s.cbar * s.rho) * (s.cbar * s.rho) + thetanew * thetanew);
-  s.cbar = s.cbar * s.rho / s.rhobar;
-  s.sbar = thetanew / s.rhobar;
-  s.zeta = s.cbar * s.zetabar;
-  s.zetabar = -s.sbar * s.zetabar;
+  const Rn alpha = s.alpha, beta = s.beta, alphabar = s.alphabar, lambda = 0.0;
+  const Rn alphahat = root(alphabar * alphabar + lambda * lambda);
+  const Rn chat = alphabar / alphahat;
+  const Rn shat = lambda / alphahat;
+  const Rn rhoold = s.rho;
+  const Rn rho = root(alphahat * alphahat + beta * beta);
+  const Rn c = alphahat / rho;
+  const Rn sn = beta / rho;
+  const Rn thetanew = sn * alpha;
+  s.alphabar = (c * alpha).v;
+  const Rn rhobarold = s.rhobar;
+  const Rn zetaold = s.zeta;
+  const Rn thetabar = Rn(s.sbar) * rho;
+  const Rn rhotemp = Rn(s.cbar) * rho;
+  const Rn rhobar = root(rhotemp * rhotemp + thetanew * thetanew);
+  const Rn cbar = rhotemp / rhobar;
+  const Rn sbar = thetanew / rhobar;
+  const Rn zeta = cbar * s.zetabar;
+  s.zetabar = (-sbar * s.zetabar).v;
+  s.rho = rho.v;
+  s.rhobar = rhobar.v;
+  s.cbar = cbar.v;
+  s.sbar = sbar.v;
+  s.zeta = zeta.v;
   // coefficients of the (deferred) vector update, lsmr.jl:138-142
-  s.c1 = -thetabar * s.rho / (rhoold * rhobarold);
-  s.c2 = s.zeta / (s.rho * s.rhobar);
-  s.c3 = -thetanew / s.rho;
+  s.c1 = (-thetabar * rho / (rhoold * rhobarold)).v;
+  s.c2 = (zeta / (rho * rhobar)).v;
+  s.c3 = (-thetanew / rho).v;
   // estimate of ||r||
-  const double betaacute = chat * s.betadd;
-  const double betacheck = -shat * s.betadd;
-  const double betahat = c * betaacute;
-  s.betadd = -sn * betaacute;
-  const double thetatildeold = s.thetatilde;
-  const double rhotildeold = sqrt(s.rhodold * s.rhodold + thetabar * thetabar);
-  const double ctildeold = s.rhodold / rhotildeold;
-  const double stildeold = thetabar / rhotildeold;
-  s.thetatilde = stildeold * s.rhobar;
-  s.rhodold = ctildeold * s.rhobar;
-  s.betad = -stildeold * s.betad + ctildeold * betahat;
-  s.tautildeold = (zetaold - thetatildeold * s.tautildeold) / rhotildeold;
-  const double taud = (s.zeta - s.thetatilde * s.tautildeold) / s.rhodold;
-  s.d = s.d + betacheck * betacheck;
-  s.normr = sqrt(s.d + (s.betad - taud) * (s.betad - taud) + s.betadd * s.betadd);
+  const Rn betaacute = chat * s.betadd;
+  const Rn betacheck = -shat * s.betadd;
+  const Rn betahat = c * betaacute;
+  const Rn betadd = -sn * betaacute;
+  const Rn thetatildeold = s.thetatilde;
+  const Rn rhotildeold = root(Rn(s.rhodold) * s.rhodold + thetabar * thetabar);
+  const Rn ctildeold = Rn(s.rhodold) / rhotildeold;
+  const Rn stildeold = thetabar / rhotildeold;
+  const Rn thetatilde = stildeold * rhobar;
+  const Rn rhodold = ctildeold * rhobar;
+  const Rn betad = -stildeold * s.betad + ctildeold * betahat;
+  const Rn tautildeold = (zetaold - thetatildeold * s.tautildeold) / rhotildeold;
+  const Rn taud = (zeta - thetatilde * tautildeold) / rhodold;
+  const Rn d = Rn(s.d) + betacheck * betacheck;
+  s.betadd = betadd.v;
+  s.thetatilde = thetatilde.v;
+  s.rhodold = rhodold.v;
+  s.betad = betad.v;
+  s.tautildeold = tautildeold.v;
+  s.d = d.v;
+  s.normr = root(d + (betad - taud) * (betad - taud) + betadd * betadd).v;
   // estimate of ||A|| and cond(A)
-  s.normA2 = s.normA2 + s.beta * s.beta;
-  s.normA = sqrt(s.normA2);
-  s.normA2 = s.normA2 + s.alpha * s.alpha;
-  s.maxrbar = s.maxrbar > rhobarold ? s.maxrbar : rhobarold;
-  if (s.iter > 1) s.minrbar = s.minrbar < rhobarold ? s.minrbar : rhobarold;
-  const double mx = s.maxrbar > rhotemp ? s.maxrbar : rhotemp;
-  const double mn = s.minrbar < rhotemp ? s.minrbar : rhotemp;
-  s.condA = mx / mn;
+  const Rn normA2 = Rn(s.normA2) + beta * beta;
+  s.normA = root(normA2).v;
+  s.normA2 = (normA2 + alpha * alpha).v;
+  s.maxrbar = s.maxrbar > rhobarold.v ? s.maxrbar : rhobarold.v;
+  if (s.iter > 1) s.minrbar = s.minrbar < rhobarold.v ? s.minrbar : rhobarold.v;
+  const double mx = s.maxrbar > rhotemp.v ? s.maxrbar : rhotemp.v;
+  const double mn = s.minrbar < rhotemp.v ? s.minrbar : rhotemp.v;
+  s.condA = (Rn(mx) / mn).v;
   s.normAr = fabs(s.zetabar);
 }
 
