@@ -546,7 +546,7 @@ static int coef_prepare(fe_plan* pl, int C, bool plain, CoefLaunch* l, CoefArgs*
   }
 
 int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int ncols,
-                    std::vector<Inst>& out, int* done) {
+                    std::vector<Inst>& out, std::vector<Inst>& start, int* done) {
   NvtxRange nv("fe: tile (coefficient side)");
   *done = 0;
   int st = coef_plan(pl);
@@ -620,6 +620,7 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
   // the inner solves run in FP64: the floor of the option's FP32 value falls
   // by the ratio of the roundings
   a.rho = pl->opt_inner_rho * 1e-6;
+  a.rho_more = pl->opt_inner_rho;
   a.maxiter = rq.maxiter - 1;
   a.max_rounds = pl->opt_max_rounds;
   {
@@ -656,7 +657,7 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
   FE_CK(cudaStreamSynchronize(pl->stream));
   uint32_t bar[3];
   memcpy(bar, res.data(), sizeof(bar));
-  if (bar[1] | bar[2]) return prof_flush(pl);
+  if (bar[1]) return prof_flush(pl);
   out.resize((size_t)C);
   memcpy(out.data(), res.data() + 64, (size_t)C * sizeof(Inst));
   // bytes of the solve kernel: per iteration (the longest column's) the index
@@ -675,8 +676,44 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
   }
   pl->prof.bytes_per_launch["coef_solve"] =
       (per + 9.0 * rn * rc) * (double)(iters + rounds) + (double)N * C * es * (1 + nf) + (double)N * rc * nf;
-  *done = 1;
+  if (bar[2] == 0) *done = 1;
+  else if (rounds > 0) start = out;
   return prof_flush(pl);
+}
+
+// X64 of one FE: the table's coefficients in the scaled unknowns of the
+// absorbed operator, for the columns of the mask
+static __global__ void k_start(const double* __restrict__ tab, const double* __restrict__ scale,
+                               double* __restrict__ x, int64_t n, int C, uint32_t mask) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n * C) return;
+  const double s = scale[e / C];
+  if ((mask >> (e % C)) & 1u) x[e] = s > 0 ? tab[e] / s : 0.0;
+}
+
+int coef_start(fe_plan* pl, int C, const std::vector<Inst>& start, double* X64,
+               std::vector<Inst>& h) {
+  const CoefPlan& cp = *pl->coef;
+  uint32_t mask = 0;
+  for (int j = 0; j < C; ++j) {
+    const Inst& s = start[(size_t)j];
+    if (s.outer_rounds < 1) continue;
+    mask |= 1u << j;
+    h[(size_t)j].outer_rounds = s.outer_rounds;
+    h[(size_t)j].iter_total = s.iter_total;
+    h[(size_t)j].normA2_prev = s.normA2_prev;
+    h[(size_t)j].normb0 = s.normb0;
+  }
+  for (int f = 0; f < cp.nf; ++f) {
+    const int k = cp.fe[f];
+    const int64_t n = pl->nlev[k];
+    if (n == 0) continue;
+    k_start<<<grid1(n * C), 256, 0, pl->stream>>>(cp.xx.as<double>() + cp.base[f] * C,
+                                                  pl->d_abs_scale_d[k].as<double>(),
+                                                  X64 + pl->lev_base[k] * C, n, C, mask);
+    FE_CK(cudaGetLastError());
+  }
+  return 0;
 }
 
 // ---------------------------------------------------------------------------

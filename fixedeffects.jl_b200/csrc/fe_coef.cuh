@@ -141,10 +141,10 @@ struct alignas(16) CoefSmem {
   double tot[3][C];
   // per column: cS, cV, cP (v update), c1, c2, c3 (deferred update), s_v
   double sc[7][C];
-  double svp[C], irr[C], nb2[C], nall[C], dt2[C];
+  double svp[C], irr[C], nb2[C], nall[C], dt2[C], t2[C];
   int vact[C], mode[C];
   Inst inst[C];
-  int ok, status;
+  int ok;
 };
 
 // norms of this CTA -> its slot of the partial buffer (`par` alternates, so a
@@ -572,6 +572,37 @@ struct CoefRowYP {
     }
   }
 };
+// ||M b||^2 from the projected rows: nrm += w (y - x_p zb)^2
+template <int C, int W>
+struct CoefRowB {
+  static constexpr int kGathers = 1, kI = 0, kD = W;
+  const float* y;
+  const double* zb;
+  const CoefSide& sd;
+  double (&nrm)[CoefShape<C>::VEC];
+  CoefRow<C> z;  // the level's
+  using Val = CoefRow<C>;
+  __device__ __forceinline__ void level(int l) {
+    if (l >= 0) z.load(zb + (int64_t)l * C);
+  }
+  __device__ __forceinline__ const int32_t* idx_array(int) const { return nullptr; }
+  __device__ __forceinline__ const double* dbl_array(int i) const { return i ? sd.dwx : sd.dw; }
+  template <int P>
+  __device__ __forceinline__ void load(const int32_t*, uint32_t i, uint32_t qa, Val& v) const {
+    v.load(y + (int64_t)(qa + i) * C);
+  }
+  template <int P>
+  __device__ __forceinline__ void add(const double* sw, uint32_t i, uint32_t, const Val& v,
+                                      CoefRow<C>&) const {
+    const double w = coef_weight<W, P>(sw, sd.dw ? 0 : -1, i);
+    const double xp = W == 2 && w != 0.0 ? coef_weight<2, P>(sw, sd.dwx ? 1 : -1, i) / w : 1.0;
+#pragma unroll
+    for (int e = 0; e < CoefShape<C>::VEC; ++e) {
+      const double u = v.v[e] - xp * z.v[e];
+      nrm[e] = fma(W ? w * u : u, u, nrm[e]);
+    }
+  }
+};
 // another FE's side of M b: s += c_y y - c_z zb
 template <int C, int W>
 struct CoefRowYF {
@@ -620,8 +651,8 @@ struct CoefRowYF {
 // The scalar step of lsmr.jl:113-186 (lambda = 0) with one reciprocal per
 // rotation, and the tests of the iteration: an inner solve ends when the outer
 // test is expected to pass, when the bidiagonalisation is exhausted, or at the
-// limit of iterations.  (The reference's atol and btol are 0 here, so its
-// tests on ||r|| hold only for a fit that is exact to rounding.)
+// limit of iterations.  (The reference's atol and btol are 0 here; of its tests
+// on ||r|| the one against ||b|| is kept, for fits that are exact.)
 template <int C>
 __device__ __forceinline__ bool coef_rotate(CoefSmem<C>& sm, int j) {
   Inst& s = sm.inst[j];
@@ -670,7 +701,8 @@ __device__ __forceinline__ bool coef_rotate(CoefSmem<C>& sm, int j) {
   const double th = s.inner_theta_tol * s.inner_theta_tol;
   return s.iter >= s.maxiter || !(mn > s.ctol * mx) ||
          !(nar2 > th * (s.normA2_prev + normA2) * normr2) ||
-         !(s.normAr > s.inner_rho * s.normAr0) || !(normr2 > 1e-32 * s.normb * s.normb);
+         !(s.normAr > s.inner_rho * s.normAr0) || !(normr2 > 1e-32 * s.normb * s.normb) ||
+         !(normr2 > th * s.normb0 * s.normb0);
 }
 
 // beta_{k+1} from T = v_k'N v_k (see fe_coef.h)
@@ -712,14 +744,20 @@ __device__ void coef_alpha(CoefSmem<C>& sm, int j) {
 }
 
 // The outer test on FP64 norms (nr2 = ||r||^2, ng = ||B'r||, nx = ||x||), and
-// the start of the next inner solve on the correction problem.
+// the start of the next inner solve on the correction problem.  True: the
+// column is beyond what this side can tell, the tile goes to the row side,
+// which forms r and goes on from x (after outer_rounds = 0: from the start):
+//   ||r||^2 = ||M b||^2 - x'(c + g) cancels when the fit is nearly exact;
+//   g = c - N x is rounding when the tolerance lies near it (another round
+//   gained less than a digit).
 template <int C>
-__device__ void coef_outer(CoefSmem<C>& sm, int j, double nr2, double ng, double nx) {
+__device__ bool coef_outer(CoefSmem<C>& sm, int j, double nr2, double ng, double nx,
+                           double rho_more) {
   Inst& s = sm.inst[j];
   sm.mode[j] = 0;
   sm.vact[j] = 0;
   s.active = 0;
-  if (!s.outer_active) return;
+  if (!s.outer_active) return false;
   const double nr = sqrt(nr2);
   if (s.outer_rounds == 0) {
     s.normb0 = nr;
@@ -729,27 +767,21 @@ __device__ void coef_outer(CoefSmem<C>& sm, int j, double nr2, double ng, double
   } else {
     s.iter_total += s.iter;
     if (s.iter > 0) s.normA2_prev += s.normA;  // (a square, see coef_rotate)
+    s.inner_rho = rho_more;
   }
   const double nAt = sqrt(s.normA2_prev);
   if (!isfinite(ng) || !isfinite(sm.nall[j])) {
-    // a NaN or infinite right-hand side stops at once, not converged
-    if (s.outer_rounds == 0) {
-      s.last_test2 = nr * ng;
-      s.converged = 0;
-    } else {
-      sm.status = (int)kCoefFallback;
+    if (s.outer_rounds > 0) {
+      s.outer_rounds = 0;
+      return true;
     }
+    // a NaN or infinite right-hand side stops at once, not converged
+    s.last_test2 = nr * ng;
+    s.converged = 0;
     s.outer_active = 0;
-    return;
+    return false;
   }
-  // ||r||^2 = ||M b||^2 - x'(c + g) and g = c - N x cancel when the fit is
-  // nearly exact; such a problem is left to the row-side path, which forms r
-  // (a zero column is not one)
-  if (!(nr2 > 1e-9 * sm.nall[j]) && sm.nall[j] != 0.0) {
-    sm.status = (int)kCoefFallback;
-    s.outer_active = 0;
-    return;
-  }
+  if (s.outer_rounds > 0 && !(nr2 > 1e-9 * sm.nb2[j])) return true;
   bool conv = false;
   s.last_test2 = (nAt > 0 && nr > 0) ? ng / (nAt * nr) : (ng == 0.0 ? 0.0 : 1.0);
   if (ng == 0.0 || nr == 0.0) {
@@ -758,13 +790,15 @@ __device__ void coef_outer(CoefSmem<C>& sm, int j, double nr2, double ng, double
     const double rtol = s.tol_b + s.tol_a * nAt * nx / s.normb0;
     conv = s.last_test2 <= s.tol_a || nr / s.normb0 <= rtol;
   }
-  if (conv || s.iter_total >= s.maxiter_total || s.outer_rounds >= s.max_rounds) {
+  if (conv || s.iter_total >= s.maxiter_total) {
     s.converged = conv ? 1 : 0;
     s.outer_active = 0;
-    // the refinement stalled above a tolerance near the rounding of c - N x
-    if (!conv && s.iter_total < s.maxiter_total) sm.status = (int)kCoefFallback;
-    return;
+    return false;
   }
+  if (s.outer_rounds >= s.max_rounds || (s.outer_rounds > 0 && s.last_test2 < 1e-15) ||
+      (s.outer_rounds > 1 && s.last_test2 > 0.1 * sm.t2[j]))
+    return true;
+  sm.t2[j] = s.last_test2;
   s.outer_rounds += 1;
   s.mode_inner = 1;
   s.maxiter = s.maxiter_total - s.iter_total;
@@ -778,6 +812,7 @@ __device__ void coef_outer(CoefSmem<C>& sm, int j, double nr2, double ng, double
   sm.sc[6][j] = s.s_v;
   sm.svp[j] = 0.0;
   sm.irr[j] = 1.0;
+  return false;
 }
 
 // ---------------------------------------------------------------------------
@@ -846,6 +881,19 @@ __device__ __noinline__ void coef_pass_yp(const CoefArgs& a, CoefSmem<C>& sm, in
 #pragma unroll
   for (int v = 0; v < VEC; ++v) nrm[0][v] += nrm[1][v];
   coef_publish<C, 2>(nrm, sm, a.part, par);
+}
+
+// ||M b||^2 as a sum over the projected rows
+template <int C, int NG, int W>
+__device__ __noinline__ void coef_pass_b(const CoefArgs& a, CoefSmem<C>& sm, int par) {
+  const int jl = (threadIdx.x & 31) % CoefShape<C>::CL;
+  const CoefSide& sd = a.p;
+  double nrm[1][CoefShape<C>::VEC];
+  coef_clear<C>(nrm);
+  coef_sweep<C, NG, W>(
+      a, sd, CoefRowB<C, W>{a.y + coef_col0<C>(jl), a.zb + coef_col0<C>(jl), sd, nrm[0], {}}, nrm,
+      coef_epi<1>(sd.lev, [](int, const auto&, CoefRow<C>&, int, auto&) {}));
+  coef_publish<C, 1>(nrm, sm, a.part, par);
 }
 
 // c = A_r'M b, the first v (into t), x = 0; norms: ||v||^2, and of two-FE
@@ -1019,10 +1067,7 @@ __global__ void __launch_bounds__(kCoefThreads, kCoefCtas<C, NG, W>()) k_coef(co
   __shared__ CoefArgs a;
   CoefSmem<C>& sm = *reinterpret_cast<CoefSmem<C>*>(coef_dyn);
   const int tid = threadIdx.x;
-  if (tid == 0) {
-    a = args;
-    sm.status = 0;
-  }
+  if (tid == 0) a = args;
   uint32_t gen = 0;
   int par = 0;
   if (tid < C) {
@@ -1042,32 +1087,51 @@ __global__ void __launch_bounds__(kCoefThreads, kCoefCtas<C, NG, W>()) k_coef(co
   double* t = a.ta;
   double* tp = a.tb;
   double nr2 = 0.0;  // thread j < C: ||M b_j||^2
+  bool handed = false;  // the row side goes on with the tile
   coef_pass_yp<C, NG, W>(a, sm, par);
   bool alive = coef_barrier(a, gen, &sm.ok);
   if (alive) {
     coef_totals<C, 2>(sm, a, par, a.multi_p, a.nmulti);
     par ^= 1;
+    // ||M b||^2 = ||b||^2 - ... loses digits where the primary FE explains most
+    // of b (a large mean): the projected rows are summed instead.  What is left
+    // of a column that is constant within the levels is rounding.
+    bool small = false;
     if (tid < C) {
       nr2 = sm.tot[0][tid];
-      sm.nall[tid] = sm.tot[1][tid];
+      const double nall = sm.nall[tid] = sm.tot[1][tid];
+      small = isfinite(nall) && nall > 0.0 && !(nr2 > 1e-4 * nall);
     }
+    if (__syncthreads_or(small)) {
+      coef_pass_b<C, NG, W>(a, sm, par);
+      alive = coef_barrier(a, gen, &sm.ok);
+      if (alive) coef_totals<C, 1>(sm, a, par, a.multi_p, a.nmulti);
+      par ^= 1;
+      if (alive && small) nr2 = sm.tot[0][tid];
+      handed = __syncthreads_or(alive && small && !(nr2 > 1e-24 * sm.nall[tid]));
+    }
+  }
+  if (alive && !handed) {
     coef_pass_yf<C, NG, W>(a, sm, t, par);
     alive = coef_barrier(a, gen, &sm.ok);
     if (alive) coef_totals<C, 2>(sm, a, par, 0, a.multi_p);
   }
   bool have_z = false;
-  while (alive) {
+  while (alive && !handed) {
     // outer test
     par ^= 1;
+    bool hand = false;
     if (tid < C) {
       if (!have_z) {
-        coef_outer<C>(sm, tid, nr2, sqrt(sm.tot[0][tid]), 0.0);
+        hand = coef_outer<C>(sm, tid, nr2, sqrt(sm.tot[0][tid]), 0.0, a.rho_more);
         sm.dt2[tid] = sm.tot[1][tid];
       } else {
-        coef_outer<C>(sm, tid, sm.nb2[tid] - sm.tot[2][tid], sqrt(sm.tot[0][tid]),
-                      sqrt(sm.tot[1][tid]));
+        hand = coef_outer<C>(sm, tid, sm.nb2[tid] - sm.tot[2][tid], sqrt(sm.tot[0][tid]),
+                             sqrt(sm.tot[1][tid]), a.rho_more);
       }
     }
+    handed = __syncthreads_or(hand);
+    if (handed) break;
     const bool outer = __syncthreads_or(tid < C && sm.inst[tid].outer_active);
     if (!outer && have_z) break;
     bool any = __syncthreads_or(tid < C && sm.inst[tid].active);
@@ -1134,7 +1198,7 @@ __global__ void __launch_bounds__(kCoefThreads, kCoefCtas<C, NG, W>()) k_coef(co
   }
   if (blockIdx.x == 0) {
     if (tid < C) a.inst[tid] = sm.inst[tid];
-    if (tid == 0 && sm.status) a.bar[2] = kCoefFallback;
+    if (tid == 0 && handed) a.bar[2] = kCoefHandOver;
   }
 }
 

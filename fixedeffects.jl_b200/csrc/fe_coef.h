@@ -92,7 +92,8 @@ struct CoefArgs {
   uint32_t* bar;             // [0] arrivals, [1] a wait gave up, [2] status
   uint32_t spins;            // polls of a grid barrier before a wait gives up
   Inst* inst;
-  double tol, theta, rho;
+  double tol, theta;
+  double rho, rho_more;      // drop of ||A'r|| that ends the first, a later inner solve
   int64_t maxiter;
   int32_t max_rounds;
 };
@@ -109,7 +110,7 @@ struct PlainArgs {
 };
 
 // status word of a solve that came to its end (bar[1] == 0): bar[2]
-constexpr uint32_t kCoefFallback = 1;  // take the row-side path instead
+constexpr uint32_t kCoefHandOver = 1;  // the row side goes on from x (coef_start)
 
 // Per-plan data of the path: index and weight arrays in every FE's level
 // order, built on the first solve that takes it, weights again after
@@ -145,9 +146,14 @@ struct CoefPlan {
 // whether the request takes the coefficient-side path
 bool coef_takes(const fe_plan* pl, const SolveReq& rq, int C);
 // one tile; *done = 0: the caller runs the row-side path (the columns are
-// untouched)
+// untouched), from the state in `start` if there is one
 int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int ncols,
-                    std::vector<Inst>& out, int* done);
+                    std::vector<Inst>& out, std::vector<Inst>& start, int* done);
+// Makes `start` the row side's state of a tile: X64 ([P][C], zero) and the
+// counts and norms of the instances h.  Columns without a finished round start
+// from zero.
+int coef_start(fe_plan* pl, int C, const std::vector<Inst>& start, double* X64,
+               std::vector<Inst>& h);
 
 // Whether a plain FP64 solve of C columns runs its loop in one kernel, and the
 // loop: the instances at `inst` (device) hold the state after the first

@@ -140,21 +140,25 @@ int solve(fe_plan* pl, const SolveReq& rq) {
     }
     return 0;
   }
-  std::vector<Inst> res;
+  std::vector<Inst> res, start;
   for (int64_t col0 = 0; col0 < ncols;) {
     const int C = tile_width(pl, ncols - col0);
     const int nc = (int)std::min<int64_t>(C, ncols - col0);
     int st;
     if (rq.before_tile && (st = rq.before_tile(rq.hook_ctx, col0, nc))) return st;
     int done = 0;
-    if (coef_takes(pl, rq, C) && (st = coef_solve_tile(pl, rq, C, col0, nc, res, &done))) return st;
+    start.clear();
+    if (coef_takes(pl, rq, C) && (st = coef_solve_tile(pl, rq, C, col0, nc, res, start, &done)))
+      return st;
+    SolveReq tile = rq;
+    if (!start.empty()) tile.start = &start;
     if (!done) switch (C) {
-      case 1: st = solve_tile_C<1>(pl, rq, col0, nc, res); break;
-      case 2: st = solve_tile_C<2>(pl, rq, col0, nc, res); break;
-      case 4: st = solve_tile_C<4>(pl, rq, col0, nc, res); break;
-      case 8: st = solve_tile_C<8>(pl, rq, col0, nc, res); break;
-      case 16: st = solve_tile_C<16>(pl, rq, col0, nc, res); break;
-      default: st = solve_tile_C<32>(pl, rq, col0, nc, res); break;
+      case 1: st = solve_tile_C<1>(pl, tile, col0, nc, res); break;
+      case 2: st = solve_tile_C<2>(pl, tile, col0, nc, res); break;
+      case 4: st = solve_tile_C<4>(pl, tile, col0, nc, res); break;
+      case 8: st = solve_tile_C<8>(pl, tile, col0, nc, res); break;
+      case 16: st = solve_tile_C<16>(pl, tile, col0, nc, res); break;
+      default: st = solve_tile_C<32>(pl, tile, col0, nc, res); break;
     }
     if (!done && st) return st;
     if (rq.after_tile && (st = rq.after_tile(rq.hook_ctx, col0, nc))) return st;

@@ -3,6 +3,8 @@
 
 #include <stdint.h>
 
+#include <vector>
+
 #include "fe_plan.h"
 
 namespace fe {
@@ -27,6 +29,8 @@ struct SolveReq {
   int (*before_tile)(void* ctx, int64_t col0, int ncols) = nullptr;
   int (*after_tile)(void* ctx, int64_t col0, int ncols) = nullptr;
   void* hook_ctx = nullptr;
+  // state of a tile that the coefficient side handed over (coef_start)
+  const std::vector<Inst>* start = nullptr;
 };
 
 // column-tile width of the next tile when `remaining` columns are left

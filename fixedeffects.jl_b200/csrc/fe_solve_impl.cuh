@@ -1708,6 +1708,9 @@ static int solve_mixed_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int n
   if (absorb && (st = tune_firm_atomic<C>(pl, c, &c.firm_atomic))) return st;
   std::vector<Inst> h;
   init_insts(pl, rq, C, ncols, h);
+  // a tile that the coefficient side has begun: its x, rounds and iterations
+  const bool begun = absorb && rq.start;
+  if (begun && (st = coef_start(pl, C, *rq.start, w.X64.as<double>(), h))) return st;
   FE_CK(cudaMemcpyAsync(c.inst, h.data(), h.size() * sizeof(Inst), cudaMemcpyHostToDevice, c.s));
   if ((st = load_tile<C>(pl, c, rq, col0, ncols))) return st;
   float* U = w.U.as<float>();
@@ -1758,7 +1761,7 @@ static int solve_mixed_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int n
     // r = b - A (x64 + dx32) in FP64, with the FP32 copy as the next inner u
     // (absorbed: r = M (b - A_r x), projected and copied by the demean pass)
     // absorbed: round 0 starts from x = 0, so r0 = M b comes straight from b
-    const bool from_b = absorb && round == 0;
+    const bool from_b = absorb && round == 0 && !begun;
     // absorbed rounds after the first, FE_OPT_FUSED_RESID: the residual and
     // its projection in one pass, by the demean kernel (2, and the default
     // where it fits) or by the staged fused kernel (1)
