@@ -382,7 +382,7 @@ int fe_plan_set_option(fe_plan* plan, int32_t option, double value) {
         set_error("inner rho must be in (0, 1)");
         return FE_ERR_INVALID;
       }
-      plan->opt_inner_rho = value;
+      plan->opt_inner_rho = plan->opt_coef_rho = value;
       return FE_OK;
     case FE_OPT_FUSE:
       plan->opt_fuse = value != 0 ? 1 : 0;

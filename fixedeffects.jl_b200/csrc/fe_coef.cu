@@ -617,9 +617,7 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
   a.inst = reinterpret_cast<Inst*>(static_cast<char*>(cp.bar.p) + 64);
   a.tol = rq.tol;
   a.theta = pl->opt_inner_theta;
-  // the inner solves run in FP64: the floor of the option's FP32 value falls
-  // by the ratio of the roundings
-  a.rho = pl->opt_inner_rho * 1e-6;
+  a.rho = pl->opt_coef_rho;
   a.rho_more = pl->opt_inner_rho;
   a.maxiter = rq.maxiter - 1;
   a.max_rounds = pl->opt_max_rounds;

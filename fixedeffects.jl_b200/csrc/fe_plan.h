@@ -232,7 +232,8 @@ struct fe_plan {
   int32_t opt_check_every = 4; // iterations between host convergence checks
   int32_t opt_max_rounds = 8;  // mixed-precision refinement rounds
   int32_t opt_unroll = 0;      // reserved
-  double opt_inner_rho = 1e-8;
+  double opt_inner_rho = 1e-8;  // drop of ||A'r|| that ends an FP32 inner solve
+  double opt_coef_rho = 1e-14;  // the same of the coefficient side's first, FP64 inner solve
   double opt_inner_theta = 0.5;
   int32_t opt_fuse = 1;        // row-sum pass: primary and small FEs reduced contiguously
   int32_t opt_ex_variant = -1; // expand kernel variant (-1: tuned default)

@@ -62,7 +62,10 @@ extern "C" {
 #define FE_OPT_CHECK_EVERY 2 /* LSMR iterations between host convergence checks */
 #define FE_OPT_MAX_ROUNDS 3  /* FP64 refinement rounds (FE_PREC_MIXED) */
 #define FE_OPT_PROFILE 4     /* 1: time every launch with CUDA events */
-#define FE_OPT_INNER_RHO 5   /* FP32 inner-solve floor (relative ||A'r|| drop) */
+#define FE_OPT_INNER_RHO 5   /* an inner solve of FE_PREC_MIXED ends at this relative
+                                drop of ||A'r||.  Default: the floor of its arithmetic,
+                                1e-8 in FP32 and 1e-14 for the first, FP64 inner solve
+                                on the coefficient side; a value set here holds for both */
 #define FE_OPT_FUSE 6        /* 1 (default): 32-column tiles of single-problem plans
                                 reduce the primary FE and up to two small FEs in one
                                 contiguous row-sum pass; 0: every FE by the
