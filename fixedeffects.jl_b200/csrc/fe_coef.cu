@@ -421,6 +421,11 @@ static bool every_row_has_levels(const fe_plan* pl) {
   return true;
 }
 
+// An option that names a kernel of the launched loops selects those.
+static bool options_allow(const fe_plan* pl) {
+  return pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0 && pl->opt_rowsum_variant < 0;
+}
+
 // Mixed-precision residual solves of FP32 columns on plans whose primary FE is
 // absorbed, with at most kCoefMaxFE other FEs, unless an option names a kernel
 // of the row-side loop.  (FP64 columns keep the row-side iteration: theirs are
@@ -432,8 +437,8 @@ bool coef_takes(const fe_plan* pl, const SolveReq& rq, int C) {
   return C <= kCoefMaxCols && rq.precision == 1 && rq.dtype == 1 && rq.residuals && pl->absorbable && pl->opt_absorb != 0 &&
          pl->opt_abs_scale != 0 && pl->nprob == 1 && !pl->xchg && pl->N > 0 &&
          pl->K - 1 <= kCoefMaxFE && pl->perm_identity[pl->primary] && pl->opt_exdm != 0 &&
-         pl->opt_exdm_pipe < 0 && pl->opt_firm_atomic == 0 && pl->opt_fused_resid != 1 &&
-         pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0 && every_row_has_levels(pl) &&
+         pl->opt_exdm_pipe < 0 && pl->opt_firm_atomic == 0 && pl->opt_fused_resid < 0 &&
+         options_allow(pl) && every_row_has_levels(pl) &&
          coef_pays(pl, C);
 }
 
@@ -724,7 +729,7 @@ int coef_start(fe_plan* pl, int C, const std::vector<Inst>& start, double* X64,
 bool plain_takes(const fe_plan* pl, const SolveReq& rq, int C) {
   return pl->N * C <= 2'500'000 && C <= kCoefMaxCols && rq.precision == 0 && pl->nprob == 1 && !pl->xchg && pl->N > 0 &&
          pl->K >= 2 && pl->K - 1 <= kCoefMaxFE && pl->perm_identity[pl->primary] &&
-         pl->opt_ex_variant < 0 && pl->opt_seg_variant < 0 && every_row_has_levels(pl);
+         options_allow(pl) && every_row_has_levels(pl);
 }
 
 int plain_loop(fe_plan* pl, int C, Inst* inst, double* U, double* V, double* H, double* Hb,

@@ -54,10 +54,11 @@ extern "C" {
 /* plan options (fe_plan_set_option).  Mixed-precision residual solves of FP32
  * columns, in tiles of up to 8, run in one kernel on the coefficient side where
  * that is measured to pay, and plain FP64 solves of small problems run their
- * loop in one kernel; FE_OPT_EXPAND_VARIANT, _SEGSUM_VARIANT (both), _ABSORB = 0,
- * _ABSORB_SCALE = 0, _FUSED_DEMEAN = 0, _EXDM_PIPE >= 0, _FIRM_ATOMIC != 0 and
- * _FUSED_RESID = 1 (the first) name kernels of the launched loops and select
- * those. */
+ * loop in one kernel.  FE_OPT_EXPAND_VARIANT, _SEGSUM_VARIANT and _ROWSUM_VARIANT
+ * >= 0 select the launched loops for both; _ABSORB = 0, _ABSORB_SCALE = 0,
+ * _FUSED_DEMEAN = 0, _EXDM_PIPE >= 0, _FIRM_ATOMIC != 0 and _FUSED_RESID >= 0
+ * for the first.  _GRAPH and _CHECK_EVERY are about the launched loops alone: a
+ * loop in one kernel is one launch and tests every iteration. */
 #define FE_OPT_TILE 1        /* column-tile width cap: 0 auto (<=32), 1,2,4,..,32 */
 #define FE_OPT_CHECK_EVERY 2 /* LSMR iterations between host convergence checks */
 #define FE_OPT_MAX_ROUNDS 3  /* FP64 refinement rounds (FE_PREC_MIXED) */

@@ -27,3 +27,36 @@ def test_inner_rho_ends_the_inner_solves_of_the_coefficient_side(fe):
     assert "coef_solve" in feM.kernel_stats()
     feM.close()
     assert np.linalg.norm(r - r0) < 1e-6 * np.linalg.norm(r0)
+
+
+@pytest.mark.parametrize("T,kernel,options", [
+    (np.float32, "coef_solve",
+     [("EXPAND_VARIANT", 0), ("SEGSUM_VARIANT", 0), ("ROWSUM_VARIANT", 1),
+      ("ABSORB", 0), ("ABSORB_SCALE", 0), ("FUSED_DEMEAN", 0), ("EXDM_PIPE", 0),
+      ("FIRM_ATOMIC", 1), ("FUSED_RESID", 0), ("FUSED_RESID", 1), ("FUSED_RESID", 2)]),
+    (np.float64, "plain_loop",
+     [("EXPAND_VARIANT", 0), ("SEGSUM_VARIANT", 0), ("ROWSUM_VARIANT", 0)])])
+def test_options_that_name_launched_kernels_select_them(fe, T, kernel, options):
+    feM, y = _solver(fe, T)
+    r0, _, _ = feM.solve_residuals(y.copy(), tol=1e-8)
+    assert kernel in feM.kernel_stats()
+    feM.close()
+    for name, value in options:
+        feM, _ = _solver(fe, T)
+        feM.set_option(getattr(fe._lib, "FE_OPT_" + name), value)
+        r, _, cv = feM.solve_residuals(y.copy(), tol=1e-8)
+        assert cv and kernel not in feM.kernel_stats(), name
+        feM.close()
+        assert np.linalg.norm(r - r0) < 1e-6 * np.linalg.norm(r0)
+
+
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+def test_graph_replay_of_the_launched_loops_matches_direct_launches(fe, T):
+    out = []
+    for graph in (1, 0):
+        feM, y = _solver(fe, T)
+        for name, value in (("PROFILE", 0), ("ROWSUM_VARIANT", 1), ("GRAPH", graph)):
+            feM.set_option(getattr(fe._lib, "FE_OPT_" + name), value)
+        out += [feM.solve_residuals(y.copy(), tol=1e-8) for _ in range(2)]
+        feM.close()
+    assert all(np.array_equal(r, out[0][0]) and it == out[0][1] for r, it, _ in out)
