@@ -52,7 +52,7 @@ int create_common(fe_plan** out, int32_t nprob, const int64_t* n_obs, int32_t K,
   pl->xchg_ctx = xchg_ctx;
   int st = 0;
   {
-    fe::StreamScope scope(&pl->stream);
+    fe::StreamScope scope(&pl->stream, !xchg);
     st = fe::plan_build(pl, nprob, n_obs, K, refs, n_levels, interaction, weights, device);
   }
   if (st) {
@@ -188,7 +188,7 @@ int solve_common(fe_plan* plan, void* Y, void* const* cols, int32_t dtype, int64
     return FE_ERR_INVALID;
   }
   if (ncols == 0) return FE_OK;
-  fe::StreamScope scope(&plan->stream);
+  fe::StreamScope scope(&plan->stream, !plan->xchg);
   const size_t es = dtype == FE_DTYPE_F64 ? 8 : 4;
   fe::SolveReq rq;
   rq.dtype = dtype;
@@ -535,7 +535,7 @@ int fe_solve_coefficients(fe_plan* plan, const void* y, int32_t dtype, int32_t p
     set_error("cudaSetDevice failed");
     return FE_ERR_CUDA;
   }
-  fe::StreamScope scope(&plan->stream);
+  fe::StreamScope scope(&plan->stream, !plan->xchg);
   const int64_t N = plan->N;
   const size_t es = dtype == FE_DTYPE_F64 ? 8 : 4;
   fe::SolveReq rq;

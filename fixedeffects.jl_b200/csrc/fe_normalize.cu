@@ -177,7 +177,7 @@ extern "C" int fe_normalize_coefficients(fe_plan* plan, double* const* coefs,
   cudaStream_t s = plan->stream;
   const int64_t N = plan->N, P = plan->P;
   if (N == 0) return FE_OK;
-  StreamScope scope(&plan->stream);
+  StreamScope scope(&plan->stream, !plan->xchg);
   DevBuf par, used, sum, cnt, mj, m, flag, mx;
   std::vector<DevBuf> dcoef(K);
   int st = par.ensure((size_t)P * 4);
@@ -293,7 +293,7 @@ extern "C" int fe_full_coefficients(fe_plan* plan, const double* const* coefs,
   if (N == 0) return FE_OK;
   FE_CK(cudaSetDevice(plan->device));
   cudaStream_t s = plan->stream;
-  StreamScope scope(&plan->stream);
+  StreamScope scope(&plan->stream, !plan->xchg);
   DevBuf dc, dout;
   for (int k = 0; k < K; ++k) {
     const int64_t n = plan->nlev[k];

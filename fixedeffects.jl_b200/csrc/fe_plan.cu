@@ -87,7 +87,10 @@ static const DevicePool* device_pool(int dev) {
 }
 
 static thread_local const StreamScope* t_scope = nullptr;
-StreamScope::StreamScope(const cudaStream_t* s) : stream(s), outer(t_scope) { t_scope = this; }
+StreamScope::StreamScope(const cudaStream_t* s, bool pool)
+    : stream(s), pooled(pool), outer(t_scope) {
+  t_scope = this;
+}
 StreamScope::~StreamScope() { t_scope = outer; }
 
 void wait_stream(cudaStream_t s) {
@@ -152,7 +155,7 @@ int DevBuf::ensure(size_t n) {
     return 3;  // FE_ERR_ALLOC
   }
   cudaError_t e = cudaErrorMemoryAllocation;
-  if (n <= kPoolBlock && t_scope) {
+  if (n <= kPoolBlock && t_scope && t_scope->pooled) {
     const int dev = current_device();
     if (const DevicePool* dp = device_pool(dev)) {
       e = cudaMallocFromPoolAsync(&p, n, dp->pool, dp->stream);
@@ -452,7 +455,7 @@ int plan_build(fe_plan* pl, int32_t nprob, const int64_t* n_obs, int32_t K,
 // update_weights!: src/SolverCPU.jl:67-76, ext/CUDAExt.jl:112-121.
 int plan_update_weights(fe_plan* pl, const double* weights) {
   NvtxRange nv("fe: weights and preconditioner");
-  StreamScope scope(&pl->stream);
+  StreamScope scope(&pl->stream, !pl->xchg);
   const int64_t N = pl->N;
   const int K = pl->K;
   cudaStream_t s = pl->stream;

@@ -87,13 +87,16 @@ void wait_stream(cudaStream_t s);
 // captures a graph on it is an error that also ends that capture.  Work on
 // other streams (the copies of a host solve, the caller's stream of
 // fe_plan_scales_noalloc) is waited for, or ordered before the plan's stream,
-// where it is queued.
+// where it is queued.  pooled = false (sharded plans): every block is a
+// cudaMalloc of its own, which the exchange callback may share with other
+// processes and GPUs as it does with any such memory; pool memory cannot be.
 struct StreamScope {
-  explicit StreamScope(const cudaStream_t* s);
+  explicit StreamScope(const cudaStream_t* s, bool pooled = true);
   ~StreamScope();
   StreamScope(const StreamScope&) = delete;
   StreamScope& operator=(const StreamScope&) = delete;
   const cudaStream_t* stream;
+  bool pooled;
   const StreamScope* outer;
 };
 

@@ -180,9 +180,10 @@ int fe_plan_create_batch(fe_plan** out, int32_t n_problems, const int64_t* n_obs
  * Observation sharding of one problem over several GPUs (one process per GPU).
  *
  * fe_exchange_fn: replaces the `count` elements at `buf` (device memory of
- * the plan's device; dtype FE_XCHG_F64 or FE_XCHG_F32) with their elementwise
- * sum over all ranks, ordered on `stream` (a cudaStream_t; completing the sum
- * before returning also satisfies the ordering).  Returns 0 on success; a
+ * the plan's device, in a cudaMalloc allocation; dtype FE_XCHG_F64 or
+ * FE_XCHG_F32) with their elementwise sum over all ranks, ordered on `stream`
+ * (a cudaStream_t; completing the sum before returning also satisfies the
+ * ordering).  Returns 0 on success; a
  * non-zero return fails the library call with FE_ERR_CUDA.  Every rank's
  * plan calls it the same number of times in the same order with the same
  * counts, as long as every rank makes the same library calls with the same
