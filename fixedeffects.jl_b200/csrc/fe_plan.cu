@@ -132,45 +132,59 @@ int exchange(fe_plan* pl, void* buf, int64_t count, int elem_bytes, cudaStream_t
   }
   return 0;
 }
-// Host-side fault injection for the allocation-failure path: with
-// FE_B200_FAIL_ALLOC_BYTES=b in the environment, every device allocation of at
-// least b bytes fails as an out-of-memory cudaMalloc would (FE_ERR_ALLOC and
-// a message), without touching the GPU.  Read on every allocation, so a test
-// can set and clear it between calls.
+// Host-side fault injection for the allocation-failure paths, without touching
+// the GPU.  FE_B200_FAIL_ALLOC_BYTES=b: every device allocation of at least b
+// bytes fails as an out-of-memory cudaMalloc would (FE_ERR_ALLOC and a
+// message); b/k: only the k-th of them since the variable has this value.
+// FE_B200_FAIL_POOL_BYTES=b: every pool request of at least b bytes fails (it
+// asks for more than any device has).  Read on every allocation, so a test can
+// set and clear them between calls.
+static std::mutex g_fail_mutex;
 static bool injected_alloc_failure(size_t n) {
+  static std::string last;
+  static long seen = 0;
   const char* v = getenv("FE_B200_FAIL_ALLOC_BYTES");
   if (!v || !*v) return false;
   char* end = nullptr;
   const unsigned long long b = strtoull(v, &end, 10);
-  return end != v && (unsigned long long)n >= b;
+  if (end == v || (unsigned long long)n < b) return false;
+  if (*end != '/') return true;
+  std::lock_guard<std::mutex> lock(g_fail_mutex);
+  if (last != v) {
+    last = v;
+    seen = 0;
+  }
+  return ++seen == strtol(end + 1, nullptr, 10);
+}
+static size_t pool_request(size_t n) {
+  const char* v = getenv("FE_B200_FAIL_POOL_BYTES");
+  if (!v || !*v || (unsigned long long)n < strtoull(v, nullptr, 10)) return n;
+  return (size_t)1 << 60;
 }
 
 int DevBuf::ensure(size_t n) {
   if (n <= bytes && p) return 0;
   release();
   if (n == 0) n = 16;
-  if (injected_alloc_failure(n)) {
-    set_error(std::string("cudaMalloc of ") + std::to_string(n) +
-              " bytes failed: injected by FE_B200_FAIL_ALLOC_BYTES");
-    return 3;  // FE_ERR_ALLOC
-  }
-  cudaError_t e = cudaErrorMemoryAllocation;
-  if (n <= kPoolBlock && t_scope && t_scope->pooled) {
-    const int dev = current_device();
-    if (const DevicePool* dp = device_pool(dev)) {
-      e = cudaMallocFromPoolAsync(&p, n, dp->pool, dp->stream);
-      if (e == cudaSuccess) {
-        pool_dev = dev;
-        e = cudaStreamSynchronize(dp->stream);
-      }
+  const bool injected = injected_alloc_failure(n);
+  const int dev = current_device();
+  const DevicePool* dp = t_scope && t_scope->pooled ? device_pool(dev) : nullptr;
+  if (dp && n <= kPoolBlock && !injected) {
+    if (cudaMallocFromPoolAsync(&p, pool_request(n), dp->pool, dp->stream) == cudaSuccess &&
+        cudaStreamSynchronize(dp->stream) == cudaSuccess) {
+      pool_dev = dev;
+      bytes = n;
+      return 0;
     }
+    // a block of its own then; the failed request must not stay behind as the
+    // error that the next launch's check finds
+    (void)cudaGetLastError();
   }
-  if (pool_dev < 0) e = cudaMalloc(&p, n);
+  cudaError_t e = injected ? cudaErrorMemoryAllocation : cudaMalloc(&p, n);
   if (e != cudaSuccess) {
-    pool_dev = -1;
     p = nullptr;
     set_error(std::string("cudaMalloc of ") + std::to_string(n) + " bytes failed: " +
-              cudaGetErrorString(e));
+              (injected ? "injected by FE_B200_FAIL_ALLOC_BYTES" : cudaGetErrorString(e)));
     (void)cudaGetLastError();
     return 3;  // FE_ERR_ALLOC
   }
