@@ -181,6 +181,12 @@ int DevBuf::ensure(size_t n) {
     (void)cudaGetLastError();
   }
   cudaError_t e = injected ? cudaErrorMemoryAllocation : cudaMalloc(&p, n);
+  if (e == cudaErrorMemoryAllocation) {
+    // what the pool keeps may be what is missing
+    (void)cudaGetLastError();
+    if (const DevicePool* kept = device_pool(dev)) cudaMemPoolTrimTo(kept->pool, 0);
+    if (!injected) e = cudaMalloc(&p, n);
+  }
   if (e != cudaSuccess) {
     p = nullptr;
     set_error(std::string("cudaMalloc of ") + std::to_string(n) + " bytes failed: " +

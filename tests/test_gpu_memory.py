@@ -23,3 +23,15 @@ def test_a_failed_pool_request_becomes_a_block_of_its_own(fe, monkeypatch, T):
     feM.close()
     assert cv and np.array_equal(r, ref)
 
+
+def test_a_failed_allocation_takes_what_the_pool_keeps(fe, monkeypatch):
+    import torch
+    fes, y = _effects(fe)
+    fe.AbstractFixedEffectSolver(fes, None, "CUDA", np.float32).close()
+    torch.cuda.synchronize()
+    kept = torch.cuda.mem_get_info()[0]
+    monkeypatch.setenv("FE_B200_FAIL_ALLOC_BYTES", "1")  # no block of the pool is in use
+    with pytest.raises(RuntimeError):
+        fe.AbstractFixedEffectSolver(fes, None, "CUDA", np.float32)
+    # the plan's refs alone were 8 x 200 kB
+    assert torch.cuda.mem_get_info()[0] > kept + (1 << 20)
