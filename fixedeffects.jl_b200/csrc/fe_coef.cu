@@ -771,6 +771,7 @@ int plain_loop(fe_plan* pl, int C, Inst* inst, double* U, double* V, double* H, 
   a.x = X;
   a.sp = cp.sp.as<double>();
   void* params[] = {&a};
+  ProfScope ps(pl, "plain_loop", 0.0);  // its bytes are known after the solve
   FE_CK(cudaLaunchCooperativeKernel(cl.kern, dim3((unsigned)cl.grid), dim3(kCoefThreads), params,
                                     cl.smem, pl->stream));
   *done = 1;

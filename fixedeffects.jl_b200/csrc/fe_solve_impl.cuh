@@ -1642,7 +1642,6 @@ static int solve_plain_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int n
   uint32_t gave_up = 0;
   if constexpr (std::is_same<T, double>::value) {
     if (one_kernel && nact > 0 && plain_takes(pl, rq, C)) {
-      ProfScope ps(pl, "plain_loop", by.expand + by.segsum + by.pupdate);
       if ((st = plain_loop(pl, C, c.inst, U, V, w.H.as<double>(), w.Hb.as<double>(), X, &in_kernel)))
         return st;
     }
@@ -1668,6 +1667,12 @@ static int solve_plain_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int n
   FE_CK(cudaMemcpyAsync(out.data(), c.inst, h.size() * sizeof(Inst), cudaMemcpyDeviceToHost, c.s));
   FE_CK(cudaStreamSynchronize(c.s));
   if (gave_up) return solve_plain_tile<T, C>(pl, rq, col0, ncols, out, false);
+  if (in_kernel) {  // the bytes of the longest column's iterations, in one launch
+    int64_t iters = 0;
+    for (const Inst& s : out) iters = std::max(iters, s.iter);
+    pl->prof.bytes_per_launch["plain_loop"] =
+        (by.expand + by.segsum + by.pupdate) * (double)std::max<int64_t>(iters, 1);
+  }
   if (!rq.residuals && rq.coefs) {
     if ((st = download_coefs<T>(pl, c, X, rq))) return st;
   }
