@@ -144,6 +144,16 @@ bool is_pinned(const void* p) {
   return a.type == cudaMemoryTypeHost;
 }
 
+// the device copy of host columns; the coefficient side's arrays make room
+int ensure_stage(fe_plan* plan, size_t n) {
+  int st = plan->ws.ystage.ensure(n);
+  if (st == FE_ERR_ALLOC && plan->coef) {
+    plan->coef.reset();
+    st = plan->ws.ystage.ensure(n);
+  }
+  return st;
+}
+
 // the plan's own stream waits for what the default stream holds now
 int order_after_default(fe_plan* plan) {
   cudaError_t e = cudaSuccess;
@@ -210,7 +220,7 @@ int solve_common(fe_plan* plan, void* Y, void* const* cols, int32_t dtype, int64
   const int64_t N = plan->N;
   HostXfer x;
   if (host && N > 0) {
-    st = plan->ws.ystage.ensure((size_t)N * ncols * es);
+    st = ensure_stage(plan, (size_t)N * ncols * es);
     if (st) return st;
     x.pl = plan;
     x.cols = cols;
@@ -554,7 +564,7 @@ int fe_solve_coefficients(fe_plan* plan, const void* y, int32_t dtype, int32_t p
   rq.prob_iters = plan->last_prob_iters.data();
   rq.prob_converged = plan->last_prob_conv.data();
   if (N > 0) {
-    st = plan->ws.ystage.ensure((size_t)N * es);
+    st = ensure_stage(plan, (size_t)N * es);
     if (st) return st;
     cudaError_t e = cudaMemcpyAsync(plan->ws.ystage.p, y, (size_t)N * es, cudaMemcpyHostToDevice,
                                     plan->stream);

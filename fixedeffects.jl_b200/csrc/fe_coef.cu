@@ -550,8 +550,8 @@ static int coef_prepare(fe_plan* pl, int C, bool plain, CoefLaunch* l, CoefArgs*
     default: { constexpr int W = 8; CALL; break; }  \
   }
 
-int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int ncols,
-                    std::vector<Inst>& out, std::vector<Inst>& start, int* done) {
+static int coef_solve(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int ncols,
+                      std::vector<Inst>& out, std::vector<Inst>& start, int* done) {
   NvtxRange nv("fe: tile (coefficient side)");
   *done = 0;
   int st = coef_plan(pl);
@@ -684,6 +684,20 @@ int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc
   return prof_flush(pl);
 }
 
+// Without room for its arrays a solve takes the launched loops, which need
+// fewer; they are given back, whole.
+static bool no_room(fe_plan* pl, int st) {
+  if (st != 3) return false;  // FE_ERR_ALLOC
+  pl->coef.reset();
+  return true;
+}
+
+int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int ncols,
+                    std::vector<Inst>& out, std::vector<Inst>& start, int* done) {
+  const int st = coef_solve(pl, rq, C, col0, ncols, out, start, done);
+  return no_room(pl, st) ? 0 : st;
+}
+
 // X64 of one FE: the table's coefficients in the scaled unknowns of the
 // absorbed operator, for the columns of the mask
 static __global__ void k_start(const double* __restrict__ tab, const double* __restrict__ scale,
@@ -742,10 +756,10 @@ int plain_loop(fe_plan* pl, int C, Inst* inst, double* U, double* V, double* H, 
   memset(&a, 0, sizeof(a));
   CoefLaunch cl;
   int st = coef_prepare(pl, C, true, &cl, &a.s);
-  if (st) return st;
-  if (!cl.grid) return 0;
-  if ((st = cp.vs.ensure((size_t)pl->P * C * 8))) return st;
-  if ((st = cp.sp.ensure((size_t)std::max<int64_t>(pl->nlev[kp], 1) * C * 8))) return st;
+  if (!st && !cl.grid) return 0;
+  if (!st) st = cp.vs.ensure((size_t)pl->P * C * 8);
+  if (!st) st = cp.sp.ensure((size_t)std::max<int64_t>(pl->nlev[kp], 1) * C * 8);
+  if (st) return no_room(pl, st) ? 0 : st;
   for (int f = 0; f <= nf; ++f) {
     CoefSide& sd = f < nf ? a.s.f[f] : a.s.p;
     const int k = f < nf ? cp.fe[f] : kp;

@@ -126,6 +126,18 @@ int tile_width(const fe_plan* pl, int64_t remaining) {
   return std::min(C, 32);
 }
 
+static int solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int nc,
+                      std::vector<Inst>& res) {
+  switch (C) {
+    case 1: return solve_tile_C<1>(pl, rq, col0, nc, res);
+    case 2: return solve_tile_C<2>(pl, rq, col0, nc, res);
+    case 4: return solve_tile_C<4>(pl, rq, col0, nc, res);
+    case 8: return solve_tile_C<8>(pl, rq, col0, nc, res);
+    case 16: return solve_tile_C<16>(pl, rq, col0, nc, res);
+    default: return solve_tile_C<32>(pl, rq, col0, nc, res);
+  }
+}
+
 int solve(fe_plan* pl, const SolveReq& rq) {
   NvtxRange nv(rq.residuals ? "fe: solve_residuals" : "fe: solve_coefficients");
   FE_CK(cudaSetDevice(pl->device));
@@ -150,17 +162,17 @@ int solve(fe_plan* pl, const SolveReq& rq) {
     start.clear();
     if (coef_takes(pl, rq, C) && (st = coef_solve_tile(pl, rq, C, col0, nc, res, start, &done)))
       return st;
-    SolveReq tile = rq;
-    if (!start.empty()) tile.start = &start;
-    if (!done) switch (C) {
-      case 1: st = solve_tile_C<1>(pl, tile, col0, nc, res); break;
-      case 2: st = solve_tile_C<2>(pl, tile, col0, nc, res); break;
-      case 4: st = solve_tile_C<4>(pl, tile, col0, nc, res); break;
-      case 8: st = solve_tile_C<8>(pl, tile, col0, nc, res); break;
-      case 16: st = solve_tile_C<16>(pl, tile, col0, nc, res); break;
-      default: st = solve_tile_C<32>(pl, tile, col0, nc, res); break;
+    if (!done) {
+      SolveReq tile = rq;
+      if (!start.empty()) tile.start = &start;
+      st = solve_tile(pl, tile, C, col0, nc, res);
+      if (st == 3 && pl->coef) {  // FE_ERR_ALLOC: without the coefficient side's arrays then
+        pl->coef.reset();
+        tile.start = nullptr;
+        st = solve_tile(pl, tile, C, col0, nc, res);
+      }
+      if (st) return st;
     }
-    if (!done && st) return st;
     if (rq.after_tile && (st = rq.after_tile(rq.hook_ctx, col0, nc))) return st;
     // per-column verdicts: a column's instances are (problem p, column j);
     // with several problems the column aggregates them (max iterations, all
