@@ -154,8 +154,16 @@ int ensure_stage(fe_plan* plan, size_t n) {
   return st;
 }
 
-// the plan's own stream waits for what the default stream holds now
+// The plan's own stream waits for what the default stream holds now.  While
+// another thread captures a stream that blocks the default stream, no call may
+// touch the latter: a solve is then ordered by its caller, who cannot queue
+// work there either.
 int order_after_default(fe_plan* plan) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(cudaStreamLegacy, &c) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
   cudaError_t e = cudaSuccess;
   if (!plan->default_order)
     e = cudaEventCreateWithFlags(&plan->default_order, cudaEventDisableTiming);

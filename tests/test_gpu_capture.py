@@ -106,3 +106,33 @@ def test_scales_on_a_callers_stream_before_the_plan_ends(fe):
     torch.cuda.synchronize()
     other.close()
     assert np.allclose(out.cpu().numpy(), ref[0], rtol=1e-13, atol=0)
+
+
+def test_a_device_solve_while_a_blocking_stream_is_captured(fe):
+    # such a capture forbids the use of the default stream to everyone; the
+    # solve runs on the plan's own stream
+    import ctypes
+    import torch
+    rt = ctypes.CDLL("libcudart.so.12")
+    fes, Y = _problem(fe, cols=1)
+    feM = fe.AbstractFixedEffectSolver(fes, None, "CUDA", np.float32)
+    y = torch.from_numpy(Y[:, 0].copy()).cuda()
+    ref = feM.solve_residuals(y.clone(), tol=1e-8)[0].cpu()
+    work = y.clone()
+    h, graph = ctypes.c_void_p(), ctypes.c_void_p()
+    buf = torch.zeros(1000, device="cuda")
+    torch.cuda.synchronize()
+    assert rt.cudaStreamCreate(ctypes.byref(h)) == 0
+    assert rt.cudaStreamBeginCapture(h, 1) == 0  # cudaStreamCaptureModeThreadLocal
+    assert rt.cudaMemsetAsync(ctypes.c_void_p(buf.data_ptr()), 0, 4000, h) == 0
+    errors, out = [], []
+    t = _thread(errors, lambda: out.append(feM.solve_residuals(work, tol=1e-8)))
+    t.join()
+    rc = rt.cudaStreamEndCapture(h, ctypes.byref(graph))
+    if rc == 0:
+        rt.cudaGraphDestroy(graph)
+    rt.cudaGetLastError()
+    rt.cudaStreamDestroy(h)
+    feM.close()
+    assert rc == 0 and not errors, (rc, errors)
+    assert torch.equal(out[0][0].cpu(), ref)
