@@ -542,6 +542,25 @@ static int coef_prepare(fe_plan* pl, int C, bool plain, CoefLaunch* l, CoefArgs*
   return 0;
 }
 
+// *fits = false: the stream's share of the GPU (a partition of its SMs) does not
+// hold the grid at once, the caller takes the launched loops.  (Host-side
+// injection, read on every launch: FE_B200_FAIL_COOPERATIVE=1 makes launches
+// fail like that.)
+static int launch_cooperative(fe_plan* pl, const CoefLaunch& l, void** params, bool* fits) {
+  const char* v = getenv("FE_B200_FAIL_COOPERATIVE");
+  const cudaError_t e =
+      v && *v == '1' ? cudaErrorCooperativeLaunchTooLarge
+                     : cudaLaunchCooperativeKernel(l.kern, dim3((unsigned)l.grid),
+                                                   dim3(kCoefThreads), params, l.smem, pl->stream);
+  *fits = e != cudaErrorCooperativeLaunchTooLarge;
+  if (!*fits) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  FE_CK(e);
+  return 0;
+}
+
 #define FE_COEF_C(C, CALL)          \
   switch (C) {                      \
     case 1: { constexpr int W = 1; CALL; break; }   \
@@ -631,12 +650,13 @@ static int coef_solve(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int 
     FE_COEF_C(C, (st = rows_in<W>(pl, rq, col0, ncols, cp.y.as<float>())));
     if (st) return st;
   }
+  bool fits = false;
   {
     ProfScope ps(pl, "coef_solve", 0.0);
     void* params[] = {&a};
-    FE_CK(cudaLaunchCooperativeKernel(cl.kern, dim3((unsigned)cl.grid), dim3(kCoefThreads), params,
-                                      cl.smem, pl->stream));
+    if ((st = launch_cooperative(pl, cl, params, &fits))) return st;
   }
+  if (!fits) return 0;
   CoefResid r;
   memset(&r, 0, sizeof(r));
   r.refp = pl->dev.refs[kp];
@@ -786,9 +806,9 @@ int plain_loop(fe_plan* pl, int C, Inst* inst, double* U, double* V, double* H, 
   a.sp = cp.sp.as<double>();
   void* params[] = {&a};
   ProfScope ps(pl, "plain_loop", 0.0);  // its bytes are known after the solve
-  FE_CK(cudaLaunchCooperativeKernel(cl.kern, dim3((unsigned)cl.grid), dim3(kCoefThreads), params,
-                                    cl.smem, pl->stream));
-  *done = 1;
+  bool fits = false;
+  if ((st = launch_cooperative(pl, cl, params, &fits))) return st;
+  *done = fits ? 1 : 0;
   return 0;
 }
 

@@ -1,6 +1,7 @@
 """Bounded waits of the cooperative solves that run out (FE_B200_SPIN_LIMIT):
 whichever of the kernel's blocks give up, the call's result is that of the
-launched loops.  Nothing hangs: every wait ends by itself.
+launched loops.  Nothing hangs: every wait ends by itself.  The same where the
+cooperative launch is refused (an error code injected on the host).
 
 The bar is the repository's 1e-6 on the residual's relative 2-norm.
 """
@@ -44,5 +45,18 @@ def test_result_does_not_depend_on_waits(fe, oracle, monkeypatch, T, limit):
     monkeypatch.delenv("FE_B200_SPIN_LIMIT")
     feM.set_option(fe._lib.FE_OPT_PROFILE, 0)
     R, _, cv = feM.solve_residuals(Y.copy(order="F"), tol=1e-8)
+    feM.close()
+    assert cv.all() and max(_rel(R[:, j], R_o[:, j]) for j in range(2)) < REL
+
+
+@pytest.mark.parametrize("T,launched", [(np.float32, "demean64"), (np.float64, "expand")])
+def test_a_grid_that_does_not_fit_takes_the_launched_loops(fe, oracle, monkeypatch, T, launched):
+    feM, Y, refs, nlev = _problem(fe, T, 2)
+    R_o, _, _ = oracle.solve_residuals_cols(Y.astype(np.float64), refs, nlev, [None] * 3, None,
+                                            tol=1e-10)
+    feM.set_option(fe._lib.FE_OPT_PROFILE, 1)
+    monkeypatch.setenv("FE_B200_FAIL_COOPERATIVE", "1")
+    R, _, cv = feM.solve_residuals(Y.copy(order="F"), tol=1e-8)
+    assert launched in feM.kernel_stats()
     feM.close()
     assert cv.all() and max(_rel(R[:, j], R_o[:, j]) for j in range(2)) < REL
