@@ -642,7 +642,7 @@ static int coef_solve(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int 
   a.tol = rq.tol;
   a.theta = pl->opt_inner_theta;
   a.rho = pl->opt_coef_rho;
-  a.rho_more = pl->opt_inner_rho;
+  a.rho_more = (float)pl->opt_inner_rho;
   a.maxiter = rq.maxiter - 1;
   a.max_rounds = pl->opt_max_rounds;
   {

@@ -141,7 +141,7 @@ struct alignas(16) CoefSmem {
   double tot[3][C];
   // per column: cS, cV, cP (v update), c1, c2, c3 (deferred update), s_v
   double sc[7][C];
-  double svp[C], irr[C], nb2[C], nall[C], dt2[C], t2[C];
+  double svp[C], irr[C], nb2[C], nall[C], dt2[C];
   int vact[C], mode[C];
   Inst inst[C];
   int ok;
@@ -796,9 +796,9 @@ __device__ bool coef_outer(CoefSmem<C>& sm, int j, double nr2, double ng, double
     return false;
   }
   if (s.outer_rounds >= s.max_rounds || (s.outer_rounds > 0 && s.last_test2 < 1e-15) ||
-      (s.outer_rounds > 1 && s.last_test2 > 0.1 * sm.t2[j]))
+      (s.outer_rounds > 1 && s.last_test2 > 0.1 * s.rd_v))
     return true;
-  sm.t2[j] = s.last_test2;
+  s.rd_v = s.last_test2;  // (of the row side's kernels, free here)
   s.outer_rounds += 1;
   s.mode_inner = 1;
   s.maxiter = s.maxiter_total - s.iter_total;

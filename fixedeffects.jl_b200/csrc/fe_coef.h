@@ -81,6 +81,7 @@ struct CoefArgs {
   CoefSide p, f[kCoefMaxFE];
   const float* y;  // sorted rows [N][C] of the right-hand sides, unweighted
   int32_t ncols;
+  uint32_t spins;            // polls of a grid barrier before a wait gives up
   double *zb, *z;            // [primary levels][C]: of b, of the current table
   double *ta, *tb;           // [levels][C]: D v_k and D v_{k-1}, unnormalised
   double *h, *hb, *x, *c;    // [levels][C]: h, hbar, x (times D); A_r'M b
@@ -90,12 +91,11 @@ struct CoefArgs {
   int32_t nmulti, multi_p;   // such levels; the primary FE's start at multi_p
   int32_t* pcnt;
   uint32_t* bar;             // [0] arrivals, [1] a wait gave up, [2] status
-  uint32_t spins;            // polls of a grid barrier before a wait gives up
   Inst* inst;
-  double tol, theta;
-  double rho, rho_more;      // drop of ||A'r|| that ends the first, a later inner solve
+  double tol, theta, rho;    // rho: drop of ||A'r|| that ends the first inner solve
   int64_t maxiter;
   int32_t max_rounds;
+  float rho_more;            // ... a later one
 };
 
 // The plain FP64 loop (fe_plain.cuh): the sides' items and scales (lev), index
