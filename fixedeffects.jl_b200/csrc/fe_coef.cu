@@ -391,24 +391,79 @@ static int rows_out(fe_plan* pl, const SolveReq& rq, int64_t col0, int ncols, fl
 // ---------------------------------------------------------------------------
 // driver
 // ---------------------------------------------------------------------------
-// Whether the passes' gathers pay: every further FE adds a gather per position
+// 0: no weights or interactions, 1: weights alone, 2: interactions
+static int entry_kind(const fe_plan* pl) {
+  int kind = pl->weighted ? 1 : 0;
+  for (int k = 0; k < pl->K; ++k)
+    if (pl->interacted[k]) kind = 2;
+  return kind;
+}
+
+// Whether the passes' gathers pay.  Every further FE adds a gather per position
 // to every other FE's pass, so their cost grows with the square of the FEs'
-// number, while the row-side loop's grows with it.  Measured, solve of the
-// row-side loop / of this one:
-//   two FEs: 10M x 1 1.78 (100k x 100 levels) and 1.04 (2M x 200k), 100M x 8 2.2
-//   three: 1M x 1 1.80, 3M x 1 1.22 and, one interacted, 1.01; 3M x 2 1.17;
-//     10M x 4 and x 8 1.02 to 1.21; 10M x 1 1.12 where the others' levels fit
-//     L1 (100 and 1000), 0.88 where they do not (200k)
-//   four: 300k x 8 1.58, 1M x 1 1.52; one interacted: 300k x 1 1.46, 1M x 1
-//     1.02, 3M x 1 0.61
+// number, while the row-side loop's grows with it; interactions add staged
+// arrays in the same way; and where levels hold two or three rows, the tables
+// (FP64, several per level) are as large as the rows they replace.  Small
+// problems gain all the same, as the row-side loop is then bound by launches.
+// The lines lie between measured ratios, solve of the row-side loop / of this
+// one, over 30k to 10M rows (to 60M for the short levels of two FEs), 1 to 8
+// columns, levels of 2 to 60 rows and FEs of few levels.  "Short" levels: fewer
+// than 2.5 (two FEs) or 3 rows per level, and 12 per level of the other FEs;
+// "long" ones: 20 rows, where the other FEs' tables do not fit L1.
+//   two FEs: 1.1 to 3.1, and below 1 for short levels of many elements only:
+//     1 column 10M 1.14, 40M 0.93, 8 columns 1M 1.13, 3M 0.94, 2 columns 40M
+//     1.16; weighted: 1 column 3M 1.24, 10M 0.96, 2 columns 10M 1.03, 4 columns 3M
+//     1.10, 10M 0.83; interacted: 1M x 4 1.03, 1M x 8 0.99, and 4 columns with
+//     long levels 1M 1.4, 3M 0.87
+//   three: 1M x 1 to x 8 1.15 to 1.6, 3M x 1 1.06 to 1.4; short levels 2M x 2
+//     1.01, 4M x 2 0.89, 3M x 4 0.93, 1M x 8 1.15, 3M x 8 0.79; 10M x 1 0.88,
+//     1.2 where the other FEs' tables fit L1; long levels 3M x 2 0.96, in L1 16M x 2 1.35;
+//     interacted: 1M x 1 1.05 to 1.36, 3M x 1 0.79 to 1.07, 300k x 2 1.11 to
+//     1.43, 1M x 2 0.76 to 0.97, 1M x 4 1.03 to 1.27, 3M x 4 0.80 to 1.03, 8
+//     columns short 300k 1.27, 1M 0.95, else 3M 1.03 to 1.08, 10M 0.93 to 1.11
+//   four: 1 column 300k 1.34 to 1.96, 1M short 0.93, else 1.0 to 1.2, 1.5M 0.98; 2
+//     columns 1M 1.07 to 1.36, 8 columns 300k 1.13 to 1.92; interacted: 1 column
+//     300k 1.23 to 1.36, 1M 0.6 to 0.8, 2 columns 300k 1.24 to 1.6, 4 columns 100k
+//     1.21 to 1.58, 8 columns 100k 1.24 to 1.42
+// "Hard" problems, of more levels than rows, or interacted with short levels in
+// three FEs, belong here whatever an iteration costs: the row side's FP32 inner
+// solves stall on them (median of 20 to 24 columns: 4M x 2 3000 iterations and
+// more against 74 here, 2M x 2 1147 against 67, 3M x 4 850 against 56, 1M x 1 of
+// four FEs 769 against 54).
 static bool coef_pays(const fe_plan* pl, int C) {
-  const int nf = pl->K - 1;
-  if (nf == 1) return true;
-  if (nf == 2)
-    return C > 2 || pl->N <= 4'000'000 || pl->P - pl->nlev[pl->primary] - pl->K <= 16'384;
-  bool inter = false;
-  for (int k = 0; k < pl->K; ++k) inter = inter || pl->interacted[k];
-  return pl->N * C <= (inter ? 1'000'000 : 2'500'000);
+  const int nf = pl->K - 1, kind = entry_kind(pl);
+  const int64_t N = pl->N, elems = N * C, levels = pl->P - pl->K;
+  int64_t largest = 0;  // of the other FEs
+  for (int k = 0; k < pl->K; ++k)
+    if (k != pl->primary) largest = std::max(largest, pl->nlev[k]);
+  const int64_t others = levels - pl->nlev[pl->primary];
+  const bool in_l1 = others <= 16'384;
+  const bool is_short = 2 * N < (nf == 1 ? 5 : 6) * levels && N < 12 * others;
+  const bool is_long = N > 20 * levels && !in_l1;
+  if (nf == 1) {
+    if (!is_short) return !(kind == 2 && C == 4 && is_long) || elems <= 6'000'000;
+    if (kind == 0) return C == 2 || elems <= 12'000'000;
+    if (kind == 1) return elems <= (C == 2 ? 24'000'000 : C == 4 ? 12'000'000 : 8'000'000);
+    return elems <= 6'000'000;
+  }
+  const bool hard =
+      levels >= N || (kind == 2 && N < 2 * levels && N < 100 * (others - largest));
+  if (nf == 2) {
+    if (C <= 2 && N > 4'000'000 && !in_l1) return false;
+    if (hard) return true;
+    if (kind < 2) {
+      if (is_short && elems > (C == 8 ? 8'000'000 : 5'000'000)) return false;
+      return !(C == 2 && is_long && N > 2'000'000);
+    }
+    if (C == 1) return N <= 1'500'000 || in_l1;
+    if (C == 2) return N <= 400'000;
+    if (C == 4) return N <= 1'500'000 || in_l1;
+    return N <= 400'000 || (!is_short && (N <= 4'000'000 || in_l1));
+  }
+  if (elems > (kind == 2 ? 1'000'000 : 2'500'000)) return false;
+  if (hard) return true;
+  if (kind < 2) return C > 1 || N <= (is_short ? 800'000 : 1'200'000);
+  return elems <= (C == 1 ? 400'000 : C == 8 ? 1'000'000 : 600'000);
 }
 
 // Both cooperative kernels follow a row to its level in every FE, so every row
@@ -480,9 +535,7 @@ struct CoefLaunch {
 static int coef_prepare(fe_plan* pl, int C, bool plain, CoefLaunch* l, CoefArgs* a) {
   CoefPlan& cp = *pl->coef;
   const int nf = cp.nf;
-  l->weights = pl->weighted ? 1 : 0;
-  for (int k = 0; k < pl->K; ++k)
-    if (pl->interacted[k]) l->weights = 2;
+  l->weights = entry_kind(pl);
   int st = coef_items(pl, C, coef_window(nf, l->weights), &l->its);
   if (st) return st;
   CoefPlan::Items* its = l->its;
@@ -756,14 +809,51 @@ int coef_start(fe_plan* pl, int C, const std::vector<Inst>& start, double* X64,
 // ---------------------------------------------------------------------------
 // the plain FP64 loop
 // ---------------------------------------------------------------------------
+// Whether the loop gains by running in one kernel, which saves launches but
+// sweeps one FE after the other, each a chain of loads (and, for an FE of few
+// levels, of pieces), where a launch sums all of them side by side.  Measured,
+// launched loop / this one, 1k to 2.4M rows, levels of 2 to 20 rows; "few": FEs of
+// few levels, 6 to 30 of them:
+//   two FEs: 1.0 to 2.0; interacted: 4 columns 10k and 30k 0.92 to 1.13, 1 column
+//     1M 1.24 to 1.39, 2.4M 0.93 to 1.18
+//   three: 1 column 1.05 to 1.7, interacted to 1M 0.99 to 1.6, 2.4M 0.86 to 1.08; 2
+//     columns 1.02 to 1.8, interacted 1.05 to 1.5, with two few 100k 1.03; 4 columns
+//     100k and more 1.2 to 1.36, with two few 100k 0.93, 300k 1.08, weighted with one
+//     few 30k 0.92, 100k 1.17; 8 columns 1.2 to 1.5, with two few 0.98, weighted 300k
+//     0.88; interacted 4 and 8 columns 0.82 to 1.19
+//   four: 1 and 2 columns 1.04 to 1.7, interacted to 300k 1.02 to 1.46, 1M 0.75 to
+//     0.97; with few 100k 0.87 to 1.1, 300k 1.12 to 1.18, 1M x 1 1.0, 1M x 2 0.97; 4
+//     and 8 columns 100k 1.19 to 1.27, 300k 1.32 to 1.52, weighted 0.93 to 1.44
+//   up to 32k rows these hold for two FEs and for 1 and 2 columns; 4 and 8 columns
+//     of three or four FEs stay here too, at 0.72 to 1.5 (up to 0.2 ms a call
+//     slower, as fast or faster below 2k rows, where one CTA runs the loop)
+// and 4M x 1 0.96, 1M x 8 0.97, 10M x 1 0.79: the bound on all of them.
+static bool plain_pays(const fe_plan* pl, int C) {
+  const int nf = pl->K - 1, kind = entry_kind(pl);
+  const int64_t N = pl->N;
+  if (N * C > 2'500'000) return false;
+  if (N <= 32'768) return true;
+  if (nf == 1) return kind < 2 || N <= 1'500'000;
+  int few = 0;
+  for (int k = 0; k < pl->K; ++k) few += k != pl->primary && 256 * pl->nlev[k] < N;
+  if (nf == 2) {
+    const bool many = few < 2 || N >= 200'000;
+    if (C == 1) return kind < 2 || N <= 1'500'000;
+    if (C == 2) return kind < 2 || many;
+    if (C == 4) return many && (kind == 0 || (kind == 1 && N >= 48'000));
+    return kind == 0 || (kind == 1 && few < 2);
+  }
+  if (few) return kind < 2 && C <= 2 && N >= 200'000 && N * C <= 1'200'000;
+  if (C <= 2) return kind < 2 || N <= 400'000;
+  return kind == 0 && N >= 80'000;
+}
+
 // One problem of two to four FEs that is bound by launches, unless an option
-// names a launched kernel of the loop.  (Launched loop / this one: 200k x 1
-// 1.32, 1M x 1 1.17 to 1.22, 2M x 1 1.11, 4M x 1 0.96, 400k x 8 1.24, 1M x 8
-// 0.97; 10M x 1 in FEs of 2M, 200k and 20 levels 0.79.)
+// names a launched kernel of the loop.
 bool plain_takes(const fe_plan* pl, const SolveReq& rq, int C) {
-  return pl->N * C <= 2'500'000 && C <= kCoefMaxCols && rq.precision == 0 && pl->nprob == 1 && !pl->xchg && pl->N > 0 &&
+  return C <= kCoefMaxCols && rq.precision == 0 && pl->nprob == 1 && !pl->xchg && pl->N > 0 &&
          pl->K >= 2 && pl->K - 1 <= kCoefMaxFE && pl->perm_identity[pl->primary] &&
-         options_allow(pl) && every_row_has_levels(pl);
+         options_allow(pl) && every_row_has_levels(pl) && plain_pays(pl, C);
 }
 
 int plain_loop(fe_plan* pl, int C, Inst* inst, double* U, double* V, double* H, double* Hb,
