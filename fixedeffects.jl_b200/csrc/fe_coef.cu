@@ -172,9 +172,11 @@ static int coef_items(fe_plan* pl, int C, int window, CoefPlan::Items** out) {
     const std::vector<int64_t>& off = pl->seg_off[k];
     const int64_t nl = pl->nlev[k];
     const double avg = nl > 0 ? std::max(1.0, (double)pl->seg_len[k] / (double)nl) : 1.0;
-    // the cheapest team size by the passes' instruction counts: a window, a
-    // round of its teams, a step of a round (a level is about two standard
-    // deviations longer than the mean where it decides the round's length)
+    // the cheapest team size by the instructions of a pass, counted in its
+    // source: a window, a round of its teams, a step of a round (a level is about
+    // two standard deviations longer than the mean where it decides the round's
+    // length).  On ten shapes (levels of 3 to 300 rows, 1 to 8 columns) its choice
+    // was within 1.5 % of the best of all sizes, the worst 1.2 to 2.8 times slower.
     const int fit = std::max(1, std::min(32, (int)(window / avg)));
     int rlog = 0, cap = fit;
     double best = 1e300;

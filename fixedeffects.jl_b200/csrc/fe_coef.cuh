@@ -8,14 +8,16 @@
 // an iteration reads the level ids (and weights) once in every FE's order and
 // gathers one row of a coefficient table per entry, from L1 or L2 unless the
 // primary FE's table outgrows them, in two passes.  Large problems are bound
-// by the passes' instructions and the latency of their gathers (1.2 warp
-// instructions per SM and cycle, 4 to 5 per row), small ones by the chain of
-// loads of a pass, the two barriers and the scalar step of an iteration (10,
-// 9 and 4 us at 800k rows).  Measured per
-// solve, against the row-side loop: 100M rows x 8 weighted columns 81.7 ->
-// 38.7 ms, 10M x 1 with three effects, one interacted, 3.7 -> 3.0 ms, 150k x 5
-// 0.91 -> 0.40 ms, 2k x 1 0.46 -> 0.15 ms, 800k x 1 of 5184 iterations 274 ->
-// 121 ms (FP64 throughout needs one inner solve where FP32 took three).
+// by the passes' instructions and the latency of their gathers (0.8 warp
+// instructions per SM and cycle, 4 to 5 per row and pass), small ones by the
+// chain of loads of a pass (of 23.6 us an iteration at 800k rows and two
+// effects the two passes take 14.1 us, averaged over the CTAs, the waits for
+// the slowest CTA and the barriers 6.0, the sums of the norms 2.4, the scalar
+// steps 1.1; in one CTA, 2k rows, 7.5, 0.2, 2.4 and 1.5 of 11.6 us).  Measured
+// per solve, against the row-side loop: 100M rows x 8 weighted columns 84.0 ->
+// 38.9 ms, 10M x 1 with three effects, one interacted, 3.4 -> 3.0 ms, 150k x 5
+// 0.91 -> 0.41 ms, 2k x 1 0.41 -> 0.14 ms, 800k x 1 of 5184 iterations 268 ->
+// 122 ms (FP64 throughout needs one inner solve where FP32 took three).
 #pragma once
 
 #include <algorithm>

@@ -1,7 +1,8 @@
 // fe_plain.cuh -- the plain FP64 LSMR loop of narrow tiles (one problem, two
 // to four fixed effects, at most 8 columns) as one cooperative kernel: the
 // iterations of src/utils/lsmr.jl:101-219 with u formed row by row, the same
-// recurrences and tests as the launched loop (fe_scalar.cu), two passes and
+// recurrences and tests as the launched loop (fe_lsmr.cuh; the norms are summed
+// in another order, so a count may differ by one), two passes and
 // two grid barriers an iteration instead of six launches:
 //   rows:    u <- s A v + c u, ||u||^2, and the primary FE's sums A_p'u, which
 //            lie in row order;
@@ -9,8 +10,8 @@
 //            by its level's update of v, h, hbar and x; the primary levels'.
 // Taken for small problems (plain_takes), which the barriers and the scalar
 // step bound; large ones are as fast launched.  Measured per solve, launched
-// loop -> this: 1M rows x 1, two effects, 0.68 -> 0.56 ms (the loop 0.53 ->
-// 0.33), the loop of 1M x 1 with three effects 0.86 -> 0.61 ms.
+// loop -> this: 1M rows x 1, two effects, 0.68 -> 0.55 ms; the loop's kernel
+// takes 0.24 ms there, 0.41 ms with three effects.
 #pragma once
 
 #include "fe_coef.cuh"

@@ -39,7 +39,8 @@ extern "C" {
 #define FE_ERR_INVALID 1 /* bad argument (lengths, level ids, null pointers) */
 #define FE_ERR_CUDA 2    /* CUDA runtime error (message in fe_last_error) */
 #define FE_ERR_ALLOC 3   /* device allocation failed */
-#define FE_ERR_TIMEOUT 4 /* a bounded device wait gave up */
+#define FE_ERR_TIMEOUT 4 /* reserved: a bounded device wait gave up (solves then run
+                            their launched loops instead) */
 
 /* precision modes (the reference's `double_precision` keyword,
  * src/AbstractFixedEffectSolver.jl:37-43) */
