@@ -754,8 +754,18 @@ static int coef_solve(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int 
   }
   pl->prof.bytes_per_launch["coef_solve"] =
       (per + 9.0 * rn * rc) * (double)(iters + rounds) + (double)N * C * es * (1 + nf) + (double)N * rc * nf;
-  if (bar[2] == 0) *done = 1;
-  else if (rounds > 0) start = out;
+  if (bar[2] == 0) {
+    *done = 1;
+    return prof_flush(pl);
+  }
+  // worth confirming if every column has been solved here, with an x that keeps
+  // r's digits, or stopped at its first test
+  bool all = true;
+  for (int j = 0; j < ncols; ++j) {
+    const Inst& s = out[(size_t)j];
+    all = all && (s.outer_rounds > 0 ? s.normx <= 1e3 * s.normb0 : !s.outer_active);
+  }
+  if (all && rounds > 0) start = out;
   return prof_flush(pl);
 }
 
@@ -791,6 +801,7 @@ int coef_start(fe_plan* pl, int C, const std::vector<Inst>& start, double* X64,
     const Inst& s = start[(size_t)j];
     if (s.outer_rounds < 1) continue;
     mask |= 1u << j;
+    h[(size_t)j].confirm = 1;
     h[(size_t)j].outer_rounds = s.outer_rounds;
     h[(size_t)j].iter_total = s.iter_total;
     h[(size_t)j].normA2_prev = s.normA2_prev;

@@ -747,14 +747,17 @@ __device__ void coef_alpha(CoefSmem<C>& sm, int j) {
 
 // The outer test on FP64 norms (nr2 = ||r||^2, ng = ||B'r||, nx = ||x||), and
 // the start of the next inner solve on the correction problem.  True: the
-// column is beyond what this side can tell, the tile goes to the row side,
-// which forms r and goes on from x (after outer_rounds = 0: from the start):
+// column is beyond what this side can tell, and the tile goes to the row side,
+// which forms r and confirms x, or solves it from the start (at once where
+// outer_rounds is left 0):
 //   ||r||^2 = ||M b||^2 - x'(c + g) cancels when the fit is nearly exact;
 //   g = c - N x is rounding when the tolerance lies near it (another round
-//   gained less than a digit).
+//   gained less than a digit);
+//   c itself is rounding, or x has grown along a direction that the data do
+//   not determine (an FE nested in another), until r would lose its digits.
 template <int C>
 __device__ bool coef_outer(CoefSmem<C>& sm, int j, double nr2, double ng, double nx,
-                           double rho_more) {
+                           double rho_more, int64_t cap) {
   Inst& s = sm.inst[j];
   sm.mode[j] = 0;
   sm.vact[j] = 0;
@@ -783,11 +786,24 @@ __device__ bool coef_outer(CoefSmem<C>& sm, int j, double nr2, double ng, double
     s.outer_active = 0;
     return false;
   }
-  if (s.outer_rounds > 0 && !(nr2 > 1e-9 * sm.nb2[j])) return true;
+  s.normx = nx;
+  if (s.outer_rounds > 0) {
+    if (!(nx <= 1e6 * s.normb0)) {
+      s.outer_rounds = 0;
+      return true;
+    }
+    if (!(nr2 > 1e-9 * sm.nb2[j])) return true;
+  } else if (ng > s.tol_a * nr && !(ng > 1e-13 * sqrt(sm.nall[j]))) {
+    return true;
+  }
   bool conv = false;
   s.last_test2 = (nAt > 0 && nr > 0) ? ng / (nAt * nr) : (ng == 0.0 ? 0.0 : 1.0);
   if (ng == 0.0 || nr == 0.0) {
     conv = true;
+  } else if (s.outer_rounds == 0) {
+    // the columns of B have norm 1 (or all but vanish), so ||B|| >= 1
+    conv = ng <= s.tol_a * nr;
+    if (conv) s.last_test2 = ng / nr;
   } else if (nAt > 0) {
     const double rtol = s.tol_b + s.tol_a * nAt * nx / s.normb0;
     conv = s.last_test2 <= s.tol_a || nr / s.normb0 <= rtol;
@@ -803,7 +819,7 @@ __device__ bool coef_outer(CoefSmem<C>& sm, int j, double nr2, double ng, double
   s.rd_v = s.last_test2;  // (of the row side's kernels, free here)
   s.outer_rounds += 1;
   s.mode_inner = 1;
-  s.maxiter = s.maxiter_total - s.iter_total;
+  s.maxiter = s.maxiter_total - s.iter_total < cap ? s.maxiter_total - s.iter_total : cap;
   s.beta = nr;
   s.u_scale = 1.0 / nr;
   s.alpha = ng / nr;
@@ -1118,6 +1134,9 @@ __global__ void __launch_bounds__(kCoefThreads, kCoefCtas<C, NG, W>()) k_coef(co
     alive = coef_barrier(a, gen, &sm.ok);
     if (alive) coef_totals<C, 2>(sm, a, par, 0, a.multi_p);
   }
+  // LSMR ends after as many iterations as there are unknowns, but for rounding;
+  // one that goes on far beyond is tested and started again
+  const int64_t cap = 4 * (a.f[NG - 1].base + a.f[NG - 1].n) + 50;
   bool have_z = false;
   while (alive && !handed) {
     // outer test
@@ -1125,11 +1144,11 @@ __global__ void __launch_bounds__(kCoefThreads, kCoefCtas<C, NG, W>()) k_coef(co
     bool hand = false;
     if (tid < C) {
       if (!have_z) {
-        hand = coef_outer<C>(sm, tid, nr2, sqrt(sm.tot[0][tid]), 0.0, a.rho_more);
+        hand = coef_outer<C>(sm, tid, nr2, sqrt(sm.tot[0][tid]), 0.0, a.rho_more, cap);
         sm.dt2[tid] = sm.tot[1][tid];
       } else {
         hand = coef_outer<C>(sm, tid, sm.nb2[tid] - sm.tot[2][tid], sqrt(sm.tot[0][tid]),
-                             sqrt(sm.tot[1][tid]), a.rho_more);
+                             sqrt(sm.tot[1][tid]), a.rho_more, cap);
       }
     }
     handed = __syncthreads_or(hand);

@@ -110,7 +110,7 @@ struct PlainArgs {
 };
 
 // status word of a solve that came to its end (bar[1] == 0): bar[2]
-constexpr uint32_t kCoefHandOver = 1;  // the row side goes on from x (coef_start)
+constexpr uint32_t kCoefHandOver = 1;  // the row side confirms x, or starts again
 
 // Per-plan data of the path: index and weight arrays in every FE's level
 // order, built on the first solve that takes it, weights again after
@@ -146,7 +146,7 @@ struct CoefPlan {
 // whether the request takes the coefficient-side path
 bool coef_takes(const fe_plan* pl, const SolveReq& rq, int C);
 // one tile; *done = 0: the caller runs the row-side path (the columns are
-// untouched), from the state in `start` if there is one
+// untouched), to confirm the state in `start` if there is one
 int coef_solve_tile(fe_plan* pl, const SolveReq& rq, int C, int64_t col0, int ncols,
                     std::vector<Inst>& out, std::vector<Inst>& start, int* done);
 // Makes `start` the row side's state of a tile: X64 ([P][C], zero) and the

@@ -164,7 +164,7 @@ struct Inst {
   int32_t pending;  // test of iteration `iter` awaits ||x||
   int32_t do_v;     // reduce updates V this iteration
   int32_t upd_mode; // deferred h/hbar/x update: 0 none, 1 init, 2 normal
-  int32_t pad0;
+  int32_t confirm;  // the outer test of a tile handed over: see PH_OUTER (fe_scalar.cu)
   // kernel coefficients
   double ex_av, ex_au;  // expand: U <- ex_av * (A V) + ex_au * U
   double rd_acc, rd_v;  // reduce: V <- rd_acc * (A'U) - rd_v * V

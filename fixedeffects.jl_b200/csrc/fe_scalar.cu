@@ -150,6 +150,11 @@ __global__ void __launch_bounds__(kScalarThreads) k_scalar(ScalarArgs a) {
         const double test1 = nr / s.normb0;
         const double rtol = s.tol_b + s.tol_a * nAt * nx / s.normb0;
         conv = (test2 <= s.tol_a) || (test1 <= rtol);
+        // a column that the coefficient side handed over: its second term lets a
+        // residual of many times the tolerance pass; no further than two
+        // roundings of the FP32 column, else the column is solved from the start
+        if (s.confirm)
+          conv = (test2 <= s.tol_a) || test1 <= fmin(rtol, fmax(s.tol_b, 1.2e-7));
       }
       if (conv) {
         s.converged = 1;

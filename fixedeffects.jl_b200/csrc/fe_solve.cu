@@ -163,11 +163,14 @@ int solve(fe_plan* pl, const SolveReq& rq) {
     if (coef_takes(pl, rq, C) && (st = coef_solve_tile(pl, rq, C, col0, nc, res, start, &done)))
       return st;
     if (!done) {
+      bool unconfirmed = false;
       SolveReq tile = rq;
+      tile.unconfirmed = &unconfirmed;
       if (!start.empty()) tile.start = &start;
       st = solve_tile(pl, tile, C, col0, nc, res);
-      if (st == 3 && pl->coef) {  // FE_ERR_ALLOC: without the coefficient side's arrays then
-        pl->coef.reset();
+      const bool no_room = st == 3 && pl->coef;  // FE_ERR_ALLOC
+      if (no_room) pl->coef.reset();
+      if (no_room || (!st && unconfirmed)) {
         tile.start = nullptr;
         st = solve_tile(pl, tile, C, col0, nc, res);
       }

@@ -29,8 +29,11 @@ struct SolveReq {
   int (*before_tile)(void* ctx, int64_t col0, int ncols) = nullptr;
   int (*after_tile)(void* ctx, int64_t col0, int ncols) = nullptr;
   void* hook_ctx = nullptr;
-  // state of a tile that the coefficient side handed over (coef_start)
+  // state of a tile that the coefficient side handed over (coef_start), whose
+  // residual is formed and tested; *unconfirmed = true: the test failed for a
+  // column, and the tile is to be solved from the start
   const std::vector<Inst>* start = nullptr;
+  bool* unconfirmed = nullptr;
 };
 
 // column-tile width of the next tile when `remaining` columns are left

@@ -1713,7 +1713,8 @@ static int solve_mixed_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int n
   if (absorb && (st = tune_firm_atomic<C>(pl, c, &c.firm_atomic))) return st;
   std::vector<Inst> h;
   init_insts(pl, rq, C, ncols, h);
-  // a tile that the coefficient side has begun: its x, rounds and iterations
+  // a tile that the coefficient side has solved but for the last test: its x,
+  // rounds and iterations
   const bool begun = absorb && rq.start;
   if (begun && (st = coef_start(pl, C, *rq.start, w.X64.as<double>(), h))) return st;
   FE_CK(cudaMemcpyAsync(c.inst, h.data(), h.size() * sizeof(Inst), cudaMemcpyHostToDevice, c.s));
@@ -1814,6 +1815,10 @@ static int solve_mixed_tile(fe_plan* pl, const SolveReq& rq, int64_t col0, int n
     int32_t nout = 0;
     if ((st = read_counter(c, 1, &nout))) return st;
     if (nout == 0) break;
+    if (begun) {
+      *rq.unconfirmed = true;
+      return prof_flush(pl);
+    }
     auto body = [&]() -> int {
       int e;
       if (absorb) {
